@@ -89,6 +89,50 @@ __device__ __forceinline__ double shape_na(int a, int i, int j, int k) {
     return a == 0 ? ni : a == 1 ? nj : a == 2 ? nk : ((1 - ni) - nj) - nk;
 }
 
+// init_f1_and_J (field_solver/device.cpp init_f1_kernel, init_J_kernel).
+__device__ __forceinline__ void init_terms(const FieldArgs& a, int64_t tid, int64_t nth) {
+    const double qe_eps0 = a.qe / a.eps0;
+    for (int64_t n = tid; n < a.n_nodes; n += nth) {
+        const int32_t e = a.node_to_eq[n];
+        if (e >= 0) a.t1[e] = qe_eps0 * (a.ion_den[n] + a.n0 * exp((a.d[e] - a.phi0) / a.kte));
+    }
+    for (int64_t u = tid; u < a.neq; u += nth) {
+        a.t2[u] = 0.0;
+        a.t3[u] = -a.qe / a.eps0 * a.n0 * exp((a.d[u] - a.phi0) / a.kte) * (1 / a.kte);
+    }
+}
+
+// build_f1_vector and build_j_matrix: per cell and unknown vertex, the 8-point integrals of
+// tempNEQ1 and tempNEQ3 times the shape function, added into F1 and tempNEQ2.
+__device__ __forceinline__ void add_cell_integrals(const FieldArgs& a, int64_t tid, int64_t nth) {
+    for (int64_t c = tid; c < a.n_cells; c += nth) {
+        const double dj = a.det_j[c];
+        for (int v = 0; v < 4; v++) {
+            const int32_t e = a.node_to_eq[a.c2n[c * 4 + v]];
+            if (e < 0) continue;
+            const double s1 = a.t1[e], s3 = a.t3[e];
+            double ff1 = 0.0, ff3 = 0.0;
+            for (int k = 0; k < 2; k++)
+                for (int j = 0; j < 2; j++)
+                    for (int i = 0; i < 2; i++) {
+                        const double na = shape_na(v, i, j, k);
+                        ff1 += s1 * na * dj * 1.0 * 1.0 * 1.0;
+                        ff3 += s3 * na * dj * 1.0 * 1.0 * 1.0;
+                    }
+            atomicAdd(a.f1 + e, ff1 * (1.0 / 8.0));
+            atomicAdd(a.t2 + e, ff3 * (1.0 / 8.0));
+        }
+    }
+}
+
+// compute_node_potential.
+__device__ __forceinline__ void node_potentials(const FieldArgs& a, int64_t tid, int64_t nth) {
+    for (int64_t n = tid; n < a.n_nodes; n += nth) {
+        const int32_t e = a.node_to_eq[n];
+        a.potential[n] = a.n_bnd_pot[n] + ((e >= 0) ? a.d[e] : 0);
+    }
+}
+
 // Row u of J v (K with its diagonal replaced by du) or, with kDiag false, of K v: four column
 // indices and values are loaded before their four vector gathers, so each thread keeps several
 // independent loads in flight; the terms are still added one by one in column order.  K is
@@ -146,39 +190,11 @@ __global__ void __launch_bounds__(kFieldBlock) field_newton_kernel(FieldArgs a) 
     __shared__ double sm[kWarps];
     const int64_t tid = (int64_t)blockIdx.x * kFieldBlock + threadIdx.x;
     const int64_t nth = (int64_t)gridDim.x * kFieldBlock;
-    const double qe_eps0 = a.qe / a.eps0;
 
-    // init_f1_and_J (field_solver/device.cpp init_f1_kernel, init_J_kernel).
-    for (int64_t n = tid; n < a.n_nodes; n += nth) {
-        const int32_t e = a.node_to_eq[n];
-        if (e >= 0) a.t1[e] = qe_eps0 * (a.ion_den[n] + a.n0 * exp((a.d[e] - a.phi0) / a.kte));
-    }
-    for (int64_t u = tid; u < a.neq; u += nth) {
-        a.t2[u] = 0.0;
-        a.t3[u] = -a.qe / a.eps0 * a.n0 * exp((a.d[u] - a.phi0) / a.kte) * (1 / a.kte);
-    }
+    init_terms(a, tid, nth);
     grid.sync();
 
-    // build_f1_vector and build_j_matrix: per cell and unknown vertex, the 8-point integrals
-    // of tempNEQ1 and tempNEQ3 times the shape function, added into F1 and tempNEQ2.
-    for (int64_t c = tid; c < a.n_cells; c += nth) {
-        const double dj = a.det_j[c];
-        for (int v = 0; v < 4; v++) {
-            const int32_t e = a.node_to_eq[a.c2n[c * 4 + v]];
-            if (e < 0) continue;
-            const double s1 = a.t1[e], s3 = a.t3[e];
-            double ff1 = 0.0, ff3 = 0.0;
-            for (int k = 0; k < 2; k++)
-                for (int j = 0; j < 2; j++)
-                    for (int i = 0; i < 2; i++) {
-                        const double na = shape_na(v, i, j, k);
-                        ff1 += s1 * na * dj * 1.0 * 1.0 * 1.0;
-                        ff3 += s3 * na * dj * 1.0 * 1.0 * 1.0;
-                    }
-            atomicAdd(a.f1 + e, ff1 * (1.0 / 8.0));
-            atomicAdd(a.t2 + e, ff3 * (1.0 / 8.0));
-        }
-    }
+    add_cell_integrals(a, tid, nth);
     grid.sync();
 
     // B = K D - F0 - F1; J's diagonal = K's - tempNEQ2; CG start x = 0, r = B, p = r / diag.
@@ -253,16 +269,317 @@ __global__ void __launch_bounds__(kFieldBlock) field_newton_kernel(FieldArgs a) 
     // D -= Y (VecAXPY(D, -1, Y)), then compute_node_potential.
     for (int64_t u = tid; u < a.neq; u += nth) a.d[u] = a.d[u] - a.x[u];
     grid.sync();
-    for (int64_t n = tid; n < a.n_nodes; n += nth) {
-        const int32_t e = a.node_to_eq[n];
-        a.potential[n] = a.n_bnd_pot[n] + ((e >= 0) ? a.d[e] : 0);
-    }
+    node_potentials(a, tid, nth);
     if (tid == 0) {
         a.status->iterations = it;
         a.status->converged = sqrt(rr) <= stop;
         a.status->resid = b_norm > 0.0 ? sqrt(rr) / b_norm : 0.0;
         a.status->b_norm = b_norm;
     }
+}
+
+// ------------------------------------------------------------- CG on K by diagonals
+//
+// The Newton step of a system stored by diagonals: two set-up kernels over the whole chip, one
+// persistent CG kernel, one kernel for the node potentials.
+//
+// What bounds the CG is neither DRAM nor arithmetic but what an iteration does one after the
+// other: grid barriers, passes over vectors in memory and the loads of K.  So each block owns a
+// contiguous range of rows and keeps x, r, q and the diagonal of its rows in registers, as many
+// diagonals of K as fit in shared memory (the others are streamed from L2), and the search
+// direction p of its rows and of the rows its diagonals reach in a shared-memory window.  Only
+// z = r / diag crosses blocks: every block forms p = z + beta p on its whole window itself (the
+// same operations on the same values in every block), which saves the third barrier.  An
+// iteration is: window update, product and p.q, reduction A, x, r and z, r.z and r.r, reduction B.
+//
+// Systems of up to kClusterNeq unknowns run as one thread-block cluster, whose barrier and
+// distributed shared memory replace the polled slots in global memory.  kCluster = false is a
+// cooperative launch of one block per SM.  At 458,591 unknowns (15 diagonals) an iteration takes
+// 14.6 us instead of 25.9 in field_newton_kernel, at 138,303 9.6 instead of 14.5.
+
+constexpr int kCgMaxThreads = 640;  // 102 registers a thread
+constexpr int kCgMaxRows = 8;       // rows a thread
+constexpr int kCgMinRows = 64;      // rows a block, where there are as many
+constexpr int kStage = 8;           // window loads in flight a thread
+constexpr int kCgMaxCluster = 16;
+constexpr int kCgMaxWarps = kCgMaxThreads / 32;
+constexpr int kCgMaxBlocks = 160;  // of the grid form
+
+constexpr int kCgSlots = (kCgMaxBlocks + 31) / 32;  // blocks' sums a lane of the polling warp reads
+constexpr int kCgMaxPolls = 1 << 20;                // about a second
+
+// One block's sums in global memory: each value and the number of the reduction it belongs to are
+// one 16-byte word, so that a block that reads the number has the value too.  A slot fills a
+// 128-byte line: every block polls every slot, and packed slots would all be served by a few L2
+// slices.
+struct __align__(16) CgWord {
+    double value;
+    unsigned long long turn;
+};
+struct __align__(128) CgSlot {
+    CgWord value[2];
+    CgWord unused[6];
+};
+
+__device__ __forceinline__ void post_word(CgWord* p, double v, unsigned long long turn) {
+    const unsigned __int128 w = ((unsigned __int128)turn << 64) | (unsigned long long)__double_as_longlong(v);
+    asm volatile("st.release.gpu.global.b128 [%0], %1;" ::"l"(p), "q"(w) : "memory");
+}
+__device__ __forceinline__ bool poll_word(const CgWord* p, unsigned long long turn, double& v) {
+    unsigned __int128 w;
+    asm volatile("ld.relaxed.gpu.global.b128 %0, [%1];" : "=q"(w) : "l"(p) : "memory");
+    v = __longlong_as_double((long long)(unsigned long long)w);
+    return (unsigned long long)(w >> 64) == turn;
+}
+
+// Reduction scratch of a block.
+struct CgShared {
+    double2 part[2][kCgMaxCluster * kCgMaxWarps];  // cluster form: the sums of every warp of the cluster
+    double2 warp[kCgMaxWarps];                     // grid form: the block's warps
+    double2 sum;
+    int failed;
+};
+
+struct CgArgs {
+    FieldArgs f;
+    int32_t rows;      // rows a block owns
+    int32_t lo, hi;    // the window reaches lo rows before and hi rows after them
+    int32_t smem_diag; // the last smem_diag diagonals are kept in shared memory
+    CgSlot* slots;     // [2][gridDim.x], grid form; zeroed before the launch
+};
+
+template <int kValues>
+__device__ __forceinline__ void warp_sum(double2& v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        v.x += __shfl_xor_sync(kFullMask, v.x, o);
+        if (kValues == 2) v.y += __shfl_xor_sync(kFullMask, v.y, o);
+    }
+}
+
+// Sum of v (its first kValues doubles) over all threads of all blocks, the same bits in every
+// thread, and a barrier of all blocks: what any thread wrote before, every thread sees after.
+// turn counts the reductions of the launch from 1.
+//
+// Cluster form: every warp stores its sum into every block's shared memory, then one cluster
+// barrier.  Grid form: the block's sum goes to its slot together with the turn, and warp 0 polls
+// the slots of all blocks, so that the reduction and the barrier are one round trip through L2
+// (a cooperative-groups grid barrier with the partial sums beside it took 7 us).  The blocks
+// are all resident (cooperative launch); a wait that runs out sets sh.failed.
+template <int kValues, bool kCluster>
+__device__ __forceinline__ double2 cg_all_sum(double2 v, CgShared& sh, CgSlot* slots, unsigned turn) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
+    const int n_blocks = (int)gridDim.x;
+    warp_sum<kValues>(v);
+    if (kCluster) {
+        double2* mine = &sh.part[turn & 1][blockIdx.x * n_warps + warp];
+        if (lane < n_blocks) *cg::this_cluster().map_shared_rank(mine, lane) = v;
+        cg::this_cluster().sync();
+        v = make_double2(0.0, 0.0);
+        for (int w = lane; w < n_blocks * n_warps; w += 32) {
+            v.x += sh.part[turn & 1][w].x;
+            if (kValues == 2) v.y += sh.part[turn & 1][w].y;
+        }
+        warp_sum<kValues>(v);
+        return v;
+    }
+    if (lane == 0) sh.warp[warp] = v;
+    __syncthreads();
+    if (warp == 0) {
+        v = lane < n_warps ? sh.warp[lane] : make_double2(0.0, 0.0);
+        warp_sum<kValues>(v);
+        CgSlot* at = slots + (turn & 1) * n_blocks;
+        if (lane == 0) {
+            __threadfence();
+            post_word(&at[blockIdx.x].value[0], v.x, turn);
+            if (kValues == 2) post_word(&at[blockIdx.x].value[1], v.y, turn);
+        }
+        double x[kCgSlots], y[kCgSlots];
+        bool all = false;
+        for (int poll = 0; !all && poll < kCgMaxPolls; poll++) {
+            bool here = true;
+#pragma unroll
+            for (int k = 0; k < kCgSlots; k++) {
+                const int b = lane + 32 * k;
+                x[k] = y[k] = 0.0;
+                if (b < n_blocks) {
+                    const bool first = poll_word(&at[b].value[0], turn, x[k]);
+                    const bool second = kValues == 1 || poll_word(&at[b].value[1], turn, y[k]);
+                    here = here && first && second;
+                }
+            }
+            all = __all_sync(kFullMask, here);
+        }
+        __threadfence();
+        v = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int k = 0; k < kCgSlots; k++) {
+            v.x += x[k];
+            if (kValues == 2) v.y += y[k];
+        }
+        warp_sum<kValues>(v);
+        if (lane == 0) {
+            sh.sum = v;
+            if (!all) sh.failed = 1;
+        }
+    }
+    __syncthreads();
+    return sh.sum;
+}
+
+template <int kRows, bool kCluster>
+__global__ void __launch_bounds__(kCgMaxThreads, 1) field_cg_kernel(const __grid_constant__ CgArgs c) {
+    extern __shared__ double dyn[];
+    __shared__ CgShared sh;
+    const FieldArgs& a = c.f;
+    const int32_t r0 = (int32_t)blockIdx.x * c.rows;
+    const int32_t n_own = max(0, min(c.rows, a.neq - r0));
+    const int32_t width = c.rows + c.lo + c.hi;
+    double* pw = dyn;          // p of rows [r0 - lo, r0 + rows + hi)
+    double* km = dyn + width;  // [smem_diag][rows]
+    double* zg = a.q;          // z of all rows, the only vector blocks exchange
+    const int32_t stream_diag = a.n_diag - c.smem_diag;
+    unsigned turn = 1;
+    if (threadIdx.x == 0) sh.failed = 0;
+    for (int32_t i = threadIdx.x; i < width; i += blockDim.x) pw[i] = 0.0;
+    for (int32_t j = 0; j < c.smem_diag; j++)
+        for (int32_t i = threadIdx.x; i < n_own; i += blockDim.x)
+            km[(int64_t)j * c.rows + i] = __ldg(a.dia_val + (int64_t)(stream_diag + j) * a.neq + r0 + i);
+
+    // B = K D - F0 - F1, J's diagonal, z = r / diag (p starts as z).
+    double x[kRows], r[kRows], dg[kRows];
+    double2 v = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int k = 0; k < kRows; k++) {
+        const int32_t i = threadIdx.x + k * blockDim.x;
+        x[k] = 0.0, r[k] = 0.0, dg[k] = 1.0;
+        if (i >= n_own) continue;
+        const int64_t u = r0 + i;
+        double kd = 0.0, kuu = 0.0;
+        for (int64_t e = __ldg(a.k_rowptr + u); e < __ldg(a.k_rowptr + u + 1); e++) {
+            const int32_t col = __ldg(a.k_col + e);
+            const double kv = __ldg(a.k_val + e);
+            kd += kv * a.d[col];
+            if (col == u) kuu = kv;
+        }
+        r[k] = (kd - a.f0[u]) - a.f1[u];
+        dg[k] = kuu + (-a.t2[u]);
+        const double z = r[k] / dg[k];
+        __stcg(zg + u, z);
+        v.x += r[k] * z;
+        v.y += r[k] * r[k];
+    }
+    v = cg_all_sum<2, kCluster>(v, sh, c.slots, turn++);
+    double rz = v.x, rr = v.y;
+    const double b_norm = sqrt(rr);
+    const double stop = fmax(a.rtol * b_norm, a.atol);
+    double beta = 0.0;
+    int it = 0;
+    while (it < a.max_iter && sqrt(rr) > stop) {
+        // p = z + beta p over the window, kStage loads of z in flight a thread.
+        for (int32_t i0 = threadIdx.x; i0 < width; i0 += kStage * blockDim.x) {
+            double z[kStage];
+#pragma unroll
+            for (int k = 0; k < kStage; k++) {
+                const int32_t i = i0 + k * blockDim.x, u = r0 - c.lo + i;
+                z[k] = i < width && (uint32_t)u < (uint32_t)a.neq ? __ldcg(zg + u) : 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < kStage; k++) {
+                const int32_t i = i0 + k * blockDim.x;
+                if (i < width) pw[i] = z[k] + beta * pw[i];
+            }
+        }
+        __syncthreads();
+        // The product, the diagonals in ascending order of their offset: each row's terms in
+        // column order.  Threads past the block's rows repeat its last one and drop the result.
+        double s[kRows];
+        int32_t row[kRows];
+#pragma unroll
+        for (int k = 0; k < kRows; k++) {
+            s[k] = 0.0;
+            row[k] = min((int32_t)(threadIdx.x + k * blockDim.x), n_own - 1);
+        }
+#pragma unroll 4
+        for (int32_t j = 0; j < stream_diag; j++) {
+            const int32_t off = a.dia_off[j];
+            const double* kj = a.dia_val + (int64_t)j * a.neq + r0;
+            const double* pj = pw + c.lo + off;
+#pragma unroll
+            for (int k = 0; k < kRows; k++) {
+                double kv = __ldg(kj + row[k]);
+                kv = off == 0 ? dg[k] : kv;
+                s[k] += kv * pj[row[k]];
+            }
+        }
+#pragma unroll 3
+        for (int32_t j = stream_diag; j < a.n_diag; j++) {
+            const int32_t off = a.dia_off[j];
+            const double* kj = km + (j - stream_diag) * c.rows;
+            const double* pj = pw + c.lo + off;
+#pragma unroll
+            for (int k = 0; k < kRows; k++) {
+                double kv = kj[row[k]];
+                kv = off == 0 ? dg[k] : kv;
+                s[k] += kv * pj[row[k]];
+            }
+        }
+        v = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int k = 0; k < kRows; k++) {
+            const int32_t i = threadIdx.x + k * blockDim.x;
+            if (i < n_own) v.x += pw[i + c.lo] * s[k];
+        }
+        v = cg_all_sum<1, kCluster>(v, sh, c.slots, turn++);
+        if (!kCluster && sh.failed) break;
+        const double alpha = rz / v.x;
+        v = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int k = 0; k < kRows; k++) {
+            const int32_t i = threadIdx.x + k * blockDim.x;
+            if (i >= n_own) continue;
+            x[k] += alpha * pw[i + c.lo];
+            r[k] = r[k] - alpha * s[k];
+            const double z = r[k] / dg[k];
+            __stcg(zg + r0 + i, z);
+            v.x += r[k] * z;
+            v.y += r[k] * r[k];
+        }
+        v = cg_all_sum<2, kCluster>(v, sh, c.slots, turn++);
+        if (!kCluster && sh.failed) break;
+        beta = v.x / rz;
+        rz = v.x;
+        rr = v.y;
+        it++;
+    }
+    const bool failed = !kCluster && sh.failed;
+    // D -= Y (VecAXPY(D, -1, Y)).
+#pragma unroll
+    for (int k = 0; k < kRows; k++) {
+        const int32_t i = threadIdx.x + k * blockDim.x;
+        if (i < n_own && !failed) a.d[r0 + i] = a.d[r0 + i] - x[k];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.status->iterations = it;
+        a.status->converged = !failed && sqrt(rr) <= stop;
+        a.status->resid = b_norm > 0.0 ? sqrt(rr) / b_norm : 0.0;
+        a.status->b_norm = b_norm;
+    }
+}
+
+__global__ void __launch_bounds__(kFieldBlock) field_init_kernel(const __grid_constant__ FieldArgs a,
+                                                                  CgSlot* slots, int n_slots) {
+    if ((int)(blockIdx.x * kFieldBlock + threadIdx.x) < n_slots)
+        slots[blockIdx.x * kFieldBlock + threadIdx.x] = CgSlot{};
+    init_terms(a, (int64_t)blockIdx.x * kFieldBlock + threadIdx.x, (int64_t)gridDim.x * kFieldBlock);
+}
+
+__global__ void __launch_bounds__(kFieldBlock) field_cells_kernel(const __grid_constant__ FieldArgs a) {
+    add_cell_integrals(a, (int64_t)blockIdx.x * kFieldBlock + threadIdx.x, (int64_t)gridDim.x * kFieldBlock);
+}
+
+__global__ void __launch_bounds__(kFieldBlock) field_potential_kernel(const __grid_constant__ FieldArgs a) {
+    node_potentials(a, (int64_t)blockIdx.x * kFieldBlock + threadIdx.x, (int64_t)gridDim.x * kFieldBlock);
 }
 
 __global__ void __launch_bounds__(256) node_charge_density_kernel(double* den, const double* vol, double spwt,
@@ -319,6 +636,126 @@ __global__ void __launch_bounds__(256) reduce_max_kernel(const double* x, int64_
         for (int w = 1; w < 8; w++) k = sm[w] > k ? sm[w] : k;
         atomicMax(&g_max_key, k);
     }
+}
+
+// How the CG on K by diagonals is launched.
+struct CgPlan {
+    int rows = 0;       // rows a block; 0 = the system does not fit this kernel
+    int blocks = 0;
+    int threads = 0;
+    int rows_thread = 0;
+    int smem_diag = 0;
+    size_t smem = 0;
+    bool cluster = false;
+};
+
+// Up to this many unknowns the CG runs as one cluster, above as one block per SM.  Microseconds an
+// iteration, cluster / grid: 4.2 / 7.3 at 4,719 unknowns, 6.1 / 7.9 at 18,207, 9.0 / 7.9 at 34,839
+// (all in field_newton_kernel: 12.9, 13.7, 13.4).
+constexpr int kClusterNeq = 24576;
+
+CgPlan cg_plan(int32_t neq, int32_t n_diag, int32_t lo, int32_t hi, int sms, int smem_max, bool cluster) {
+    CgPlan p;
+    p.cluster = cluster;
+    const int most = cluster ? kCgMaxCluster : sms < kCgMaxBlocks ? sms : kCgMaxBlocks;
+    p.rows = ceil_div(neq, most);
+    if (p.rows < kCgMinRows) p.rows = kCgMinRows;
+    p.blocks = ceil_div(neq, p.rows);
+    p.rows_thread = ceil_div(p.rows, kCgMaxThreads);
+    const int64_t window = ((int64_t)p.rows + lo + hi) * (int64_t)sizeof(double);
+    if (p.rows_thread > kCgMaxRows || window > smem_max) return CgPlan{};
+    p.threads = (ceil_div(p.rows, p.rows_thread) + 31) / 32 * 32;
+    p.smem_diag = (int)((smem_max - window) / ((int64_t)p.rows * (int64_t)sizeof(double)));
+    if (p.smem_diag > n_diag) p.smem_diag = n_diag;
+    p.smem = (size_t)(window + (int64_t)p.smem_diag * p.rows * (int64_t)sizeof(double));
+    return p;
+}
+
+template <int kRows, bool kCluster>
+int launch_cg(const CgPlan& p, CgArgs& c, cudaStream_t s) {
+    auto kernel = field_cg_kernel<kRows, kCluster>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess)
+        return OPPB_ERR_LAUNCH;
+    if (kCluster && p.blocks > 8 &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+        return OPPB_ERR_LAUNCH;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(p.blocks);
+    cfg.blockDim = dim3(p.threads);
+    cfg.dynamicSmemBytes = p.smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr{};
+    if (kCluster) {
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = (unsigned)p.blocks;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    } else {
+        attr.id = cudaLaunchAttributeCooperative;
+        attr.val.cooperative = 1;
+    }
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, c) == cudaSuccess ? OPPB_OK : OPPB_ERR_LAUNCH;
+}
+
+template <bool kCluster>
+int launch_cg_rows(const CgPlan& p, CgArgs& c, cudaStream_t s) {
+    switch (p.rows_thread) {
+        case 1: return launch_cg<1, kCluster>(p, c, s);
+        case 2: return launch_cg<2, kCluster>(p, c, s);
+        case 3: return launch_cg<3, kCluster>(p, c, s);
+        case 4: return launch_cg<4, kCluster>(p, c, s);
+        case 5: return launch_cg<5, kCluster>(p, c, s);
+        case 6: return launch_cg<6, kCluster>(p, c, s);
+        case 7: return launch_cg<7, kCluster>(p, c, s);
+        default: return launch_cg<8, kCluster>(p, c, s);
+    }
+}
+
+// The plan for this system on the current device; rows = 0 when it takes field_newton_kernel.
+int make_cg_plan(const FieldArgs& a, CgPlan* plan, int32_t* lo, int32_t* hi) {
+    *plan = CgPlan{};
+    if (a.n_diag <= 0 || a.neq <= 0) return OPPB_OK;
+    int64_t first = 0, last = 0;
+    for (int j = 0; j < a.n_diag; j++) {
+        first = a.dia_off[j] < first ? a.dia_off[j] : first;
+        last = a.dia_off[j] > last ? a.dia_off[j] : last;
+        if (j > 0 && a.dia_off[j] <= a.dia_off[j - 1]) return OPPB_OK;
+    }
+    if (-first >= a.neq || last >= a.neq) return OPPB_OK;
+    *lo = (int32_t)-first, *hi = (int32_t)last;
+    int dev = 0, sms = 0, coop = 0, smem = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+        return OPPB_ERR_LAUNCH;
+    smem -= (int)sizeof(CgShared) + 64;  // the kernel's static part
+    if (a.neq <= kClusterNeq) *plan = cg_plan(a.neq, a.n_diag, *lo, *hi, sms, smem, true);
+    if (!plan->rows && coop) *plan = cg_plan(a.neq, a.n_diag, *lo, *hi, sms, smem, false);
+    return OPPB_OK;
+}
+
+int solve_by_diagonals(const FieldArgs& a, const CgPlan& p, int32_t lo, int32_t hi, cudaStream_t s) {
+    const int most = 148 * 8;
+    const int eq_grid = ceil_div(a.n_nodes, kFieldBlock), cell_grid = ceil_div(a.n_cells, kFieldBlock);
+    CgArgs c{};
+    c.f = a;
+    c.rows = p.rows, c.lo = lo, c.hi = hi, c.smem_diag = p.smem_diag;
+    // The slots lie in the vectors x, r and p of the work space, which this path keeps on chip:
+    // 32 doubles a block of at least kCgMinRows rows, and the alignment.
+    static_assert(3 * kCgMinRows >= 32 + 16, "the slots fit");
+    c.slots = reinterpret_cast<CgSlot*>((reinterpret_cast<uintptr_t>(a.x) + 127) & ~(uintptr_t)127);
+    const int n_slots = p.cluster ? 0 : 2 * p.blocks;
+    const int slot_grid = ceil_div(n_slots, kFieldBlock);
+    const int init_grid = eq_grid < most ? (eq_grid > slot_grid ? eq_grid : slot_grid) : most;
+    field_init_kernel<<<init_grid, kFieldBlock, 0, s>>>(a, c.slots, n_slots);
+    field_cells_kernel<<<cell_grid, kFieldBlock, 0, s>>>(a);
+    const int rc = p.cluster ? launch_cg_rows<true>(p, c, s) : launch_cg_rows<false>(p, c, s);
+    if (rc) return rc;
+    field_potential_kernel<<<eq_grid < most ? eq_grid : most, kFieldBlock, 0, s>>>(a);
+    count_launches(4);
+    return launch_status();
 }
 
 int coop_grid(int* blocks) {
@@ -408,9 +845,6 @@ extern "C" int oppb_field_solve(const oppb_field_device* f, const oppb_field_con
         return OPPB_ERR_ARG;
     if (c->max_iter < 0 || !(c->kte != 0.0) || !(c->eps0 != 0.0) || !(c->rtol >= 0.0) || !(c->atol >= 0.0))
         return OPPB_ERR_ARG;
-    int blocks = 0;
-    int rc = coop_grid(&blocks);
-    if (rc) return rc;
     const size_t n = (size_t)(f->neq > 0 ? f->neq : 1);
     double* w = f->work;
     FieldArgs a{};
@@ -428,6 +862,13 @@ extern "C" int oppb_field_solve(const oppb_field_device* f, const oppb_field_con
     a.n_diag = f->n_diag;
     for (int j = 0; j < OPPB_FIELD_MAX_DIAG; j++) a.dia_off[j] = f->dia_off[j];
     a.dia_val = f->dia_val;
+    CgPlan plan;
+    int32_t lo = 0, hi = 0;
+    int rc = make_cg_plan(a, &plan, &lo, &hi);
+    if (rc) return rc;
+    if (plan.rows) return solve_by_diagonals(a, plan, lo, hi, as_stream(stream));
+    int blocks = 0;
+    if ((rc = coop_grid(&blocks))) return rc;
     void* args[] = {&a};
     if (cudaLaunchCooperativeKernel((const void*)field_newton_kernel, dim3(blocks), dim3(kFieldBlock), args, 0,
                                     as_stream(stream)) != cudaSuccess)
