@@ -1,12 +1,15 @@
 // CabanaPIC particle hot path: relativistic Boris push, streak walk across hex-cell faces and
 // the charge-conserving current deposit into the 12 per-cell accumulators, one launch.
 //
-// One thread per particle; a particle's calls of the reference kernel (the first one with the
-// push, then one per face crossing) run in a warp-wide loop so that every call's deposit goes
-// through one warp reduction: lanes whose deposits target the same cell are summed in shared
-// memory and each such group issues 12 FP64 atomics.  Particles are initialised cell by cell
-// and move a few hundredths of a cell per step, so a warp's lanes spread over a few cells and
-// the reduction turns 384 atomics per warp into a few dozen.
+// One thread per particle for the push.  About 6 % of a two-stream step's particles cross a face, so
+// almost every warp holds one or two of them, and the streak walk run in place costs the whole warp its
+// length: they are queued in shared memory instead and walked by the block's first warps, packed.
+// The 12 values that a particle adds to its start cell become one row in shared memory; the rows
+// are ordered by cell over the whole block (warp match, then a small hash table of the block's
+// cells), so that a thread sums one accumulator over a run of rows and issues one FP64 atomic per
+// cell of its run.  Bound by instruction issue and FP64 latency (the correctly rounded divides and
+// square roots).  104.9M particles of the two-stream state: 6.66 ms a call against 8.72 with the
+// walk in place, one staged reduction a warp and the visit counters added once a warp.
 //
 // FP64 expressions are written in the reference's order and this file is compiled with
 // -fmad=false (no contraction), so positions, momenta, streaks and cells are bit-identical to
@@ -267,18 +270,12 @@ __device__ __forceinline__ int streak_step(double q, double pos[3], double s[3],
     return axis + (d > 0 ? 3 : 0);
 }
 
-// Staging of one warp's deposits: 32 rows of 12 values (rows 16-B aligned).
-struct WarpStage {
-    double vals[32][kStageStride];
-    int32_t keys[32];
-};
-
 // Adds every lane's 12 values j to acc[k * acc_stride + key] (key < 0: nothing).  Lanes with
 // the same key form a group (warp match, whatever their positions: the two counter-streaming
 // species interleave lane by lane and drift apart); lanes 0..11 sum one column each over a
 // group's rows in shared memory and issue one atomic per column and group.  Every lane of
 // the warp must call it.
-__device__ __forceinline__ void warp_deposit(WarpStage& ws, double* acc, int32_t acc_stride, int32_t key,
+__device__ __forceinline__ void warp_deposit(double (*rows)[kStageStride], int32_t* keys, double* acc, int32_t acc_stride, int32_t key,
                                              const double* j) {
     const int lane = threadIdx.x & 31;
     // Calls after the first one (face crossings) involve a few lanes of a warp: their
@@ -294,10 +291,10 @@ __device__ __forceinline__ void warp_deposit(WarpStage& ws, double* acc, int32_t
     unsigned leaders = __ballot_sync(kFullMask, key >= 0 && lane == __ffs(peers) - 1);
     if (leaders == 0u) return;
     __syncwarp();  // the previous call's readers are done with the stage
-    double2* row = reinterpret_cast<double2*>(&ws.vals[lane][0]);
+    double2* row = reinterpret_cast<double2*>(rows[lane]);
 #pragma unroll
     for (int c = 0; c < 6; c++) row[c] = make_double2(j[2 * c], j[2 * c + 1]);
-    ws.keys[lane] = key;
+    keys[lane] = key;
     __syncwarp();
     while (leaders) {  // warp-uniform
         const int leader = __ffs(leaders) - 1;
@@ -308,9 +305,9 @@ __device__ __forceinline__ void warp_deposit(WarpStage& ws, double* acc, int32_t
             while (members) {
                 const int r = __ffs(members) - 1;
                 members &= members - 1;
-                sum += ws.vals[r][lane];
+                sum += rows[r][lane];
             }
-            atomicAdd(acc + (int64_t)lane * acc_stride + ws.keys[leader], sum);
+            atomicAdd(acc + (int64_t)lane * acc_stride + keys[leader], sum);
         }
     }
 }
@@ -320,31 +317,102 @@ struct ConstsF32 {
     float qdt_2mc, cdx, cdy, cdz;
 };
 
+// Shared memory of a block: one row of 12 accumulator values per particle, ordered by cell, 32
+// more rows for the face-crossing particles' later segments, and the cell groups' table.
+struct CabShared {
+    double rows[kCabBlock + 32][kStageStride];
+    int32_t row_key[kCabBlock + 32];  // the cell of every row
+    int32_t tab_key[kCabBlock];       // open-addressing table of the block's cells, -1 = free
+    int32_t tab_cnt[kCabBlock];       // rows of each, then the first row of each
+    int32_t warp_rows[kCabWarps];
+    int32_t n_cross;
+    uint16_t cross_row[kCabBlock];    // crossing particles: their row and their thread
+    uint16_t cross_thread[kCabBlock];
+};
+
+// The row of this thread's values such that the rows of one cell are contiguous: lanes of a
+// warp with the same key take their place in the key's table slot together.  key < 0: no row.
+// Sets *n_rows to the block's row count.  Every thread of the block must call it.
+__device__ __forceinline__ int cell_ordered_row(CabShared& sh, int32_t key, int* n_rows) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned peers = __match_any_sync(kFullMask, key);
+    const int leader = __ffs(peers) - 1;
+    unsigned h = 0;
+    int base = 0;
+    if (lane == leader && key >= 0) {
+        h = ((uint32_t)key * 2654435761u) >> 24;
+        for (int probe = 0; probe < kCabBlock; probe++) {  // at most kCabBlock distinct keys: one is free
+            const int32_t k = atomicCAS(&sh.tab_key[h], -1, key);
+            if (k == -1 || k == key) break;
+            h = (h + 1) & (kCabBlock - 1);
+        }
+        base = atomicAdd(&sh.tab_cnt[h], __popc(peers));
+    }
+    h = __shfl_sync(kFullMask, h, leader);
+    base = __shfl_sync(kFullMask, base, leader);
+    __syncthreads();
+    int incl = sh.tab_cnt[threadIdx.x];
+    const int own = incl;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(kFullMask, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) sh.warp_rows[warp] = incl;
+    __syncthreads();
+    int first = incl - own, total = 0;
+#pragma unroll
+    for (int w = 0; w < kCabWarps; w++) {
+        const int c = sh.warp_rows[w];
+        first += w < warp ? c : 0;
+        total += c;
+    }
+    sh.tab_cnt[threadIdx.x] = first;
+    __syncthreads();
+    *n_rows = total;
+    return sh.tab_cnt[h] + base + __popc(peers & lanemask_lt());
+}
+
+__device__ __forceinline__ void write_row(double* row, const double* j) {
+    double2* r = reinterpret_cast<double2*>(row);
+#pragma unroll
+    for (int c = 0; c < 6; c++) r[c] = make_double2(j[2 * c], j[2 * c + 1]);
+}
+
+// The neighbour through a face; -1 when the map's entry is no cell.
+__device__ __forceinline__ int32_t through_face(const HexArgs& m, int32_t cell, int face) {
+    const int32_t next = __ldg(m.c2f + (int64_t)cell * 8 + face);
+    return (uint32_t)next < (uint32_t)m.n_cells ? next : -1;
+}
+
+constexpr int kSumChunks = 10;                     // row ranges of the block's sums
+constexpr int kSumThreads = kSumChunks * 12;       // one thread per range and accumulator
+static_assert(kSumThreads <= kCabBlock - 32, "the sums fit beside the crossing particles' warp");
+
 // kOcc: resident CTAs per SM the kernel is compiled for (oppb_tuning.cabana_occupancy): 0 = the
-// compiler's register count (FP64 form 76 registers, 3 CTAs per SM; FP32-momentum form 64, 4),
-// 4 (64 registers, no spills) or 5 (48 registers, about 100 B of spills a thread).
+// compiler's register count, 4 (64 registers) or 5 (48 registers).
 template <bool kF32Mom, int kOcc>
 __global__ void __launch_bounds__(kCabBlock, kOcc > 0 ? kOcc : 1) cabana_move_deposit_kernel(HexArgs m, CabParts p,
                                                                         oppb_cabana_consts k, ConstsF32 kf,
                                                                         double* acc, int32_t acc_stride,
                                                                         oppb_move_status* st, int32_t max_hops) {
-    __shared__ __align__(16) WarpStage stage[kCabWarps];
-    const int64_t i = (int64_t)blockIdx.x * kCabBlock + threadIdx.x;
+    extern __shared__ __align__(16) unsigned char cab_smem[];
+    CabShared& sh = *reinterpret_cast<CabShared*>(cab_smem);
+    const int64_t base = (int64_t)blockIdx.x * kCabBlock;
+    const int64_t i = base + threadIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t sd = p.stride;
+    sh.tab_key[threadIdx.x] = -1;
+    sh.tab_cnt[threadIdx.x] = 0;
+    if (threadIdx.x == 0) sh.n_cross = 0;
     const bool active = i < p.size;
-    int32_t cell = active ? ld_stream(p.p2c + i) : -1;
-    const int32_t cell0 = cell;
-    int err = 0;
-    bool going = active;
-    if (going && (uint32_t)cell >= (uint32_t)m.n_cells) {
-        err = OPPB_ERR_CELL_RANGE;
-        going = false;
-    }
+    const int32_t cell = active ? ld_stream(p.p2c + i) : -1;
+    const bool pushed = active && (uint32_t)cell < (uint32_t)m.n_cells;
+    if (active && !pushed) raise_error(st, OPPB_ERR_CELL_RANGE, (int32_t)i);
     double pos[3] = {0.0, 0.0, 0.0}, u[3] = {0.0, 0.0, 0.0}, s[3] = {0.0, 0.0, 0.0};
     float uf[3] = {0.0f, 0.0f, 0.0f};
     double q = 0.0;
-    const int64_t sd = p.stride;
-    if (going) {
+    if (pushed) {
 #pragma unroll
         for (int d = 0; d < 3; d++) {
             pos[d] = ld_stream(p.pos + d * sd + i);
@@ -355,47 +423,128 @@ __global__ void __launch_bounds__(kCabBlock, kOcc > 0 ? kOcc : 1) cabana_move_de
         }
         q = __ldg(p.weight + i) * k.qsp;
     }
-    const bool pushed = going;
-    bool streaking = false;
-    int calls = 0;
-    while (__any_sync(kFullMask, going)) {
+    __syncthreads();
+    int n_rows;
+    int row = cell_ordered_row(sh, pushed ? cell : -1, &n_rows);
+
+    // The push (OPP_DO_ONCE).  A particle that stays in its cell is finished; one that leaves it
+    // queues, with its state in its row, for the streak walk by a full warp below.
+    if (pushed) {
         double j[12];
-        int32_t key = -1;
-        if (going) {
-            calls++;
-            key = cell;
-            // The first call pushes (OPP_DO_ONCE); unless the particle stays in its cell, it
-            // goes on, in the same call, with the first streak segment.
-            bool stay = false;
-            if (calls == 1) {
-                if (kF32Mom)
-                    stay = push_once_f32(m.interp32 + (int64_t)cell * 20, kf.qdt_2mc, kf.cdx, kf.cdy, kf.cdz, q, pos,
-                                         uf, s, j);
-                else
-                    stay = push_once(m.interp + (int64_t)cell * 20, k.qdt_2mc, k.cdt_d[0], k.cdt_d[1], k.cdt_d[2],
-                                     q, pos, u, s, j);
-                streaking = !stay;
+        bool stay;
+        if (kF32Mom)
+            stay = push_once_f32(m.interp32 + (int64_t)cell * 20, kf.qdt_2mc, kf.cdx, kf.cdy, kf.cdz, q, pos, uf, s, j);
+        else
+            stay = push_once(m.interp + (int64_t)cell * 20, k.qdt_2mc, k.cdt_d[0], k.cdt_d[1], k.cdt_d[2], q, pos, u,
+                             s, j);
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            if (kF32Mom)
+                __stcs(p.vel32 + d * sd + i, uf[d]);
+            else
+                st_stream(p.vel + d * sd + i, u[d]);
+        }
+        sh.row_key[row] = cell;
+        if (stay) {
+#pragma unroll
+            for (int d = 0; d < 3; d++) st_stream(p.pos + d * sd + i, pos[d]);
+            write_row(sh.rows[row], j);
+        } else {
+            const int e = atomicAdd(&sh.n_cross, 1);
+            sh.cross_row[e] = (uint16_t)row;
+            sh.cross_thread[e] = (uint16_t)threadIdx.x;
+            double* r = sh.rows[row];
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                r[d] = pos[d];
+                r[3 + d] = s[d];
             }
-            if (stay) {
-                going = false;
+            r[6] = q;
+        }
+    }
+    __syncthreads();
+
+    // The crossing particles, packed into the first warps: their first segment belongs to the
+    // cell they start in and takes their row of the block's sums.
+    const int n_cross = sh.n_cross;
+    bool going = false, crossing = (int)threadIdx.x < n_cross;
+    int32_t at = -1, from = -1;  // the particle's cell now and at the start
+    int calls = 0, err = 0;
+    int64_t ic = 0;
+    if (crossing) {
+        row = sh.cross_row[threadIdx.x];
+        ic = base + sh.cross_thread[threadIdx.x];
+        double* r = sh.rows[row];
+        at = from = sh.row_key[row];
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            pos[d] = r[d];
+            s[d] = r[3 + d];
+        }
+        q = r[6];
+        double j[12];
+        const int face = streak_step(q, pos, s, j);
+        write_row(r, j);
+        calls = 1;
+        if (face >= 0) {
+            const int32_t next = through_face(m, at, face);
+            if (next < 0) {
+                err = OPPB_ERR_CELL_RANGE;
             } else {
+                at = next;
+                going = calls < max_hops;
+                if (!going) err = OPPB_ERR_HOP_LIMIT;
+            }
+        }
+    }
+    if (n_cross > 0) __syncthreads();
+
+    // The block's sums: each thread adds one accumulator over a range of rows and issues one
+    // atomic per cell of its range.  With crossing particles warp 0 goes on with their walks.
+    const int t = (int)threadIdx.x - (n_cross > 0 ? 32 : 0);
+    if (t >= 0 && t < kSumThreads) {
+        const int c = t % 12, per = (n_rows + kSumChunks - 1) / kSumChunks;
+        int r = (t / 12) * per;
+        const int end = min(r + per, n_rows);
+        if (r < end) {
+            double* out = acc + (int64_t)c * acc_stride;
+            int32_t key = sh.row_key[r];
+            double sum = 0.0;
+#pragma unroll 4
+            for (; r < end; r++) {
+                const int32_t kr = sh.row_key[r];
+                const double v = sh.rows[r][c];
+                if (kr != key) {
+                    atomicAdd(out + key, sum);
+                    sum = 0.0;
+                    key = kr;
+                }
+                sum += v;
+            }
+            atomicAdd(out + key, sum);
+        }
+    }
+    if (n_cross > 32) __syncthreads();  // the rows are free: the other warps stage in them
+
+    // Later segments, one warp-grouped deposit a segment.
+    if (warp * 32 < n_cross) {
+        const int first = warp == 0 ? kCabBlock : warp * 32;
+        while (__any_sync(kFullMask, going)) {
+            double j[12];
+            int32_t key = -1;
+            if (going) {
+                calls++;
+                key = at;
                 const int face = streak_step(q, pos, s, j);
                 if (face < 0) {
                     going = false;
                 } else {
-                    const int4 f0 = ldg_i4(m.c2f + (int64_t)cell * 8);
-                    const int2 f1 = __ldg(reinterpret_cast<const int2*>(m.c2f + (int64_t)cell * 8 + 4));
-                    const int32_t next = face == 0 ? f0.x
-                                         : face == 1 ? f0.y
-                                         : face == 2 ? f0.z
-                                         : face == 3 ? f0.w
-                                         : face == 4 ? f1.x
-                                                     : f1.y;
-                    if ((uint32_t)next >= (uint32_t)m.n_cells) {
+                    const int32_t next = through_face(m, at, face);
+                    if (next < 0) {
                         err = OPPB_ERR_CELL_RANGE;
                         going = false;
                     } else {
-                        cell = next;
+                        at = next;
                         if (calls >= max_hops) {
                             err = OPPB_ERR_HOP_LIMIT;
                             going = false;
@@ -403,28 +552,29 @@ __global__ void __launch_bounds__(kCabBlock, kOcc > 0 ? kOcc : 1) cabana_move_de
                     }
                 }
             }
+            warp_deposit(sh.rows + first, sh.row_key + first, acc, acc_stride, key, j);
         }
-        warp_deposit(stage[warp], acc, acc_stride, key, j);
-    }
-    if (err) raise_error(st, err, (int32_t)i);
-    if (pushed) {
+        if (err) raise_error(st, err, (int32_t)ic);
+        if (crossing) {
 #pragma unroll
-        for (int d = 0; d < 3; d++) {
-            st_stream(p.pos + d * sd + i, pos[d]);
-            if (kF32Mom)
-                __stcs(p.vel32 + d * sd + i, uf[d]);
-            else
-                st_stream(p.vel + d * sd + i, u[d]);
-            if (streaking) st_stream(p.streak + d * sd + i, s[d]);
+            for (int d = 0; d < 3; d++) {
+                st_stream(p.pos + d * sd + ic, pos[d]);
+                st_stream(p.streak + d * sd + ic, s[d]);
+            }
+            if (at != from) st_stream(p.p2c + ic, at);
         }
-        if (cell != cell0) st_stream(p.p2c + i, cell);
     }
-    // Visit statistics: warp reductions in the integer unit, one atomic per counter per warp.
-    const unsigned vsum = __reduce_add_sync(kFullMask, (unsigned)calls);
-    const unsigned vmax = __reduce_max_sync(kFullMask, (unsigned)calls);
-    if (lane == 0) {
-        if (vsum) atomicAdd(reinterpret_cast<unsigned long long*>(&st->total_visits), (unsigned long long)vsum);
-        if (vmax) atomicMax(&st->max_visits, (int)vmax);
+    // Visit statistics: every pushed particle calls once, the crossing ones more often.  One
+    // atomic per counter per block (and per further crossing warp): all blocks share two words.
+    if (warp == 0 || warp * 32 < n_cross) {
+        unsigned vsum = __reduce_add_sync(kFullMask, (unsigned)max(calls - 1, 0));
+        const unsigned vmax = __reduce_max_sync(kFullMask, (unsigned)calls);
+        if (lane == 0) {
+            if (warp == 0) vsum += (unsigned)n_rows;
+            if (vsum) atomicAdd(reinterpret_cast<unsigned long long*>(&st->total_visits), (unsigned long long)vsum);
+            const int most = max((int)vmax, warp == 0 && n_rows > 0 ? 1 : 0);
+            if (most > *reinterpret_cast<volatile int32_t*>(&st->max_visits)) atomicMax(&st->max_visits, most);
+        }
     }
 }
 
@@ -505,7 +655,9 @@ int launch_cabana(const oppb_hex_mesh* mesh, const oppb_cabana_particles* parts,
     auto kernel = occ == 5   ? cabana_move_deposit_kernel<kF32Mom, 5>
                   : occ == 4 ? cabana_move_deposit_kernel<kF32Mom, 4>
                              : cabana_move_deposit_kernel<kF32Mom, 0>;
-    kernel<<<ceil_div(parts->size, kCabBlock), kCabBlock, 0, s>>>(
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CabShared)) != cudaSuccess)
+        return OPPB_ERR_LAUNCH;
+    kernel<<<ceil_div(parts->size, kCabBlock), kCabBlock, sizeof(CabShared), s>>>(
         m, p, *consts, kf, acc, acc_stride, status, max_hops);
     count_launches(1);
     return launch_status();
