@@ -32,13 +32,20 @@ __device__ __forceinline__ int find_instance(const int32_t* __restrict__ prefix,
     return cursor;
 }
 
-// update_pos_kernel for one axis: x += v dt, then the periodic wrap.
-__device__ __forceinline__ double update_axis(double x, double v, double dt, double extent) {
+// update_pos_kernel for one axis: x += v dt, then the periodic wrap by trunc(temp / extent), the
+// quotient correctly rounded.  inv = 1 / extent: where temp * inv lies at least 2^-20 from an
+// integer (its error is below 2^30 * 2^-51) the truncation is the divide's, and the divide, some
+// twenty instructions of a kernel that issue bounds as much as DRAM, is only made next to one.
+__device__ __forceinline__ double update_axis(double x, double v, double dt, double extent, double inv) {
     const double offset = v * dt;
     x += offset;
     const int n_extent_offset_int = __double2int_rz(fabs(x) + 2.0);
     const double temp_pos = x + (double)n_extent_offset_int * extent;
-    return temp_pos - extent * trunc(__ddiv_rn(temp_pos, extent));
+    const double q = temp_pos * inv;
+    double k = trunc(q);
+    const double f = q - k;
+    if (!(f > 0x1p-20 && f < 1.0 - 0x1p-20 && q < 0x1p30)) k = trunc(__ddiv_rn(temp_pos, extent));
+    return temp_pos - extent * k;
 }
 
 // move_kernel's hops for one particle; returns the number of calls, sets *err on failure.
@@ -94,32 +101,32 @@ __device__ __forceinline__ int move_particle(const double* __restrict__ cells, i
 // index instead of read from the record, which oppb_advec_check_grid found equal to them bit
 // for bit.  The walk keeps (ix, iy) and steps them with the periodic wrap; the arithmetic
 // and the decisions are move_particle's.
-__device__ __forceinline__ int move_particle_grid(int32_t nx, int32_t n_cells, double x, double y, int& mx, int& my,
-                                                  int32_t& cell, double cw, double ex, double ey, int32_t max_hops,
-                                                  int& err) {
+// inv_nx = 1 / nx: (cell + 0.5) / nx is half a cell away from an integer, so truncating the product
+// gives cell / nx.
+__device__ __forceinline__ int move_particle_grid(int32_t nx, int32_t ny, double inv_nx, int32_t n_cells, double x, double y,
+                                                  int& mx, int& my, int32_t& cell, double cw, double ex, double ey,
+                                                  int32_t max_hops, int& err) {
     if ((uint32_t)cell >= (uint32_t)n_cells) {
         err = OPPB_ERR_CELL_RANGE;
         return 0;
     }
-    const int32_t ny = n_cells / nx;
-    int32_t iy = cell / nx;
+    int32_t iy = __double2int_rz(((double)cell + 0.5) * inv_nx);
     int32_t ix = cell - iy * nx;
+    double dx = x - (double)ix * cw;  // c_pos_ll = (x * cell_width, y * cell_width)
+    double dy = y - (double)iy * cw;
+    const bool xp = ((dx > cw) && (ex > 2 * dx - cw)) || ((dx < 0) && (ex < cw - 2 * dx));
+    const bool yp = ((dy > cw) && (ey > 2 * dy - cw)) || ((dy < 0) && (ey < cw - 2 * dy));
+    mx = xp ? 1 : -1;  // OPP_DO_ONCE
+    my = yp ? 1 : -1;
     int calls = 0;
     for (;;) {
         calls++;
-        const double dx = x - (double)ix * cw;  // c_pos_ll = (x * cell_width, y * cell_width)
-        const double dy = y - (double)iy * cw;
-        if (calls == 1) {  // OPP_DO_ONCE
-            const bool xp = ((dx > cw) && (ex > 2 * dx - cw)) || ((dx < 0) && (ex < cw - 2 * dx));
-            const bool yp = ((dy > cw) && (ey > 2 * dy - cw)) || ((dy < 0) && (ey < cw - 2 * dy));
-            mx = xp ? 1 : -1;
-            my = yp ? 1 : -1;
-        }
         bool hop = false;
         if ((dx >= 0.0) && (dx <= cw)) {
             mx = 0;
         } else if (mx != 0) {
             ix = mx > 0 ? (ix + 1 >= nx ? 0 : ix + 1) : (ix - 1 < 0 ? nx - 1 : ix - 1);  // xu_y : xd_y
+            dx = x - (double)ix * cw;
             hop = true;
         }
         if (!hop) {
@@ -127,6 +134,7 @@ __device__ __forceinline__ int move_particle_grid(int32_t nx, int32_t n_cells, d
                 my = 0;
             } else if (my != 0) {
                 iy = my > 0 ? (iy + 1 >= ny ? 0 : iy + 1) : (iy - 1 < 0 ? ny - 1 : iy - 1);  // x_yu : x_yd
+                dy = y - (double)iy * cw;
                 hop = true;
             }
         }
@@ -140,7 +148,7 @@ __device__ __forceinline__ int move_particle_grid(int32_t nx, int32_t n_cells, d
     return calls;
 }
 
-constexpr int kChunkItems = 8;  // work items a block takes from the counter at once
+constexpr int kChunkItems = 8;  // work items a block takes from the counter at once, at most
 
 // Direct-hop seed (oppb_advec_dh): the cell of the grid box holding (x, y), or kRemoved
 // outside the grid or in a box without a cell.  Each box coordinate is (pos - min) * (1/h)
@@ -156,10 +164,15 @@ __device__ __forceinline__ int32_t dh_seed_2d(const oppb_advec_dh& g, double x, 
 
 // A block takes a chunk of work items from the batch's counter (so items are processed in
 // order across the whole GPU) and walks it kItems items per pass (one particle of each per
-// thread), so every thread has kItems independent particles' loads in flight.
-template <int kMode, int kItems, bool kSeed>
-__global__ void __launch_bounds__(kAdvBlock) advec_kernel(oppb_advec_batch b, oppb_move_status* st,
-                                                          int32_t max_hops) {
+// thread), so every thread has kItems independent particles' loads in flight.  kOnce: the grid
+// has a block for every chunk, which then is the block's only one and needs no counter.
+//
+// Bound by DRAM with issue close behind (665M particles: 8.70 ms a step, 75 % of the measured copy
+// bandwidth for the 64 B a particle; 9.74 with the direction read and the divides made).  The
+// move direction is not read: move_kernel's first call (OPP_DO_ONCE) overwrites it.
+template <int kMode, int kItems, bool kSeed, bool kOnce>
+__global__ void __launch_bounds__(kAdvBlock, kItems == 1 ? 5 : kItems == 2 ? 4 : 2) advec_kernel(oppb_advec_batch b, oppb_move_status* st,
+                                                          int32_t max_hops, int32_t chunk_items) {
     static_assert(kChunkItems % kItems == 0, "a chunk is a whole number of passes");
     static_assert(!kSeed || kMode != kUpdateOnly, "the seed belongs to the move");
     __shared__ int s_chunk;
@@ -167,16 +180,22 @@ __global__ void __launch_bounds__(kAdvBlock) advec_kernel(oppb_advec_batch b, op
     int my_max = 0;
     int my_removed = 0;
     int cursor = 0;
+    int params_of = -1;  // the instance whose reciprocals these are
+    double inv_ex = 0.0, inv_ey = 0.0, inv_nx = 0.0;
+    int32_t gny = 0;
     const int64_t sd = b.stride;
     for (;;) {
-        if (threadIdx.x == 0) s_chunk = atomicAdd(b.work_counter, kChunkItems);
-        __syncthreads();
-        const int chunk = s_chunk;
-        __syncthreads();
-        if (chunk >= b.n_work) break;
-        for (int w0 = chunk; w0 < chunk + kChunkItems && w0 < b.n_work; w0 += kItems) {
+        int chunk = (int)blockIdx.x * chunk_items;
+        if (!kOnce) {
+            if (threadIdx.x == 0) s_chunk = atomicAdd(b.work_counter, chunk_items);
+            __syncthreads();
+            chunk = s_chunk;
+            __syncthreads();
+            if (chunk >= b.n_work) break;
+        }
+        for (int w0 = chunk; w0 < chunk + chunk_items && w0 < b.n_work; w0 += kItems) {
             double x[kItems], y[kItems], vx[kItems], vy[kItems];
-            int32_t cell[kItems], mx[kItems], my[kItems];
+            int32_t cell[kItems];
             int64_t idx[kItems];
             int inst[kItems];
             bool ok[kItems];
@@ -195,14 +214,10 @@ __global__ void __launch_bounds__(kAdvBlock) advec_kernel(oppb_advec_batch b, op
                 x[k] = ld_stream(b.pos + i);
                 y[k] = ld_stream(b.pos + sd + i);
                 if (kMode != kMoveOnly) {
-                    vx[k] = __ldg(b.vel + i);
-                    vy[k] = __ldg(b.vel + sd + i);
+                    vx[k] = __ldcs(b.vel + i);
+                    vy[k] = __ldcs(b.vel + sd + i);
                 }
-                if (kMode != kUpdateOnly) {
-                    cell[k] = ld_stream(b.p2c + i);
-                    mx[k] = ld_stream(b.mdir + i);
-                    my[k] = ld_stream(b.mdir + sd + i);
-                }
+                if (kMode != kUpdateOnly) cell[k] = ld_stream(b.p2c + i);
             }
     #pragma unroll
             for (int k = 0; k < kItems; k++) {
@@ -210,10 +225,17 @@ __global__ void __launch_bounds__(kAdvBlock) advec_kernel(oppb_advec_batch b, op
                 const oppb_advec_instance& I = b.instances[inst[k]];
                 const int64_t i = idx[k];
                 const double ex = __ldg(&I.extents[0]), ey = __ldg(&I.extents[1]);
+                const int32_t gnx = __ldg(&I.grid_nx);
+                if (inst[k] != params_of) {
+                    params_of = inst[k];
+                    inv_ex = 1.0 / ex, inv_ey = 1.0 / ey;
+                    inv_nx = 1.0 / (double)(gnx > 0 ? gnx : 1);
+                    gny = gnx > 0 ? __ldg(&I.n_cells) / gnx : 0;
+                }
                 if (kMode != kMoveOnly) {
                     const double dt = __ldg(&I.dt);
-                    x[k] = update_axis(x[k], vx[k], dt, ex);
-                    y[k] = update_axis(y[k], vy[k], dt, ey);
+                    x[k] = update_axis(x[k], vx[k], dt, ex, inv_ex);
+                    y[k] = update_axis(y[k], vy[k], dt, ey, inv_ey);
                     st_stream(b.pos + i, x[k]);
                     st_stream(b.pos + sd + i, y[k]);
                 }
@@ -227,16 +249,17 @@ __global__ void __launch_bounds__(kAdvBlock) advec_kernel(oppb_advec_batch b, op
                             continue;
                         }
                     }
-                    int err = 0;
-                    const int32_t gnx = __ldg(&I.grid_nx);
+                    int err = 0, mx = 0, my = 0;
                     const int calls =
-                        gnx > 0 ? move_particle_grid(gnx, __ldg(&I.n_cells), x[k], y[k], mx[k], my[k], cell[k],
+                        gnx > 0 ? move_particle_grid(gnx, gny, inv_nx, __ldg(&I.n_cells), x[k], y[k], mx, my, cell[k],
                                                      __ldg(&I.cell_width), ex, ey, max_hops, err)
-                                : move_particle(b.cells, __ldg(&I.cell_offset), __ldg(&I.n_cells), x[k], y[k], mx[k],
-                                                my[k], cell[k], __ldg(&I.cell_width), ex, ey, max_hops, err);
+                                : move_particle(b.cells, __ldg(&I.cell_offset), __ldg(&I.n_cells), x[k], y[k], mx, my,
+                                                cell[k], __ldg(&I.cell_width), ex, ey, max_hops, err);
                     if (err) raise_error(st, err, (int32_t)i);
-                    st_stream(b.mdir + i, mx[k]);
-                    st_stream(b.mdir + sd + i, my[k]);
+                    if (calls > 0) {  // without a call (an invalid cell) the direction stays as it was
+                        st_stream(b.mdir + i, mx);
+                        st_stream(b.mdir + sd + i, my);
+                    }
                     // Every processed particle's cell is stored, changed or not: a warp then
                     // writes whole sectors of p2c, which DRAM takes without reading them first.
                     st_stream(b.p2c + i, cell[k]);
@@ -245,6 +268,7 @@ __global__ void __launch_bounds__(kAdvBlock) advec_kernel(oppb_advec_batch b, op
                 }
             }
         }
+        if (kOnce) break;
     }
     if (kMode == kUpdateOnly) return;
     // One atomic per counter per block: the grid is persistent, so this is a few hundred.
@@ -311,34 +335,47 @@ __global__ void __launch_bounds__(256) advec_check_grid_kernel(const double* cel
 
 // Persistent grid: resident blocks of the kernel on every SM (cached per device and variant).
 template <int kMode, int kItems, bool kSeed>
-int persistent_grid(int n_blocks_needed) {
+int resident_blocks() {
     static int cached[64] = {0};
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return n_blocks_needed;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
     if (!cached[dev]) {
         int sms = 0, per_sm = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, advec_kernel<kMode, kItems, kSeed>, kAdvBlock, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, advec_kernel<kMode, kItems, kSeed, false>, kAdvBlock,
+                                                      0);
         cached[dev] = sms * (per_sm > 0 ? per_sm : 1);
     }
-    return n_blocks_needed < cached[dev] ? n_blocks_needed : cached[dev];
+    return cached[dev];
 }
 
+// With no more chunks of kItems work items than resident blocks, every block takes one chunk by
+// its index: no counter to reset, and 8-item chunks would leave most SMs idle (538 items of one
+// 61 x 61-cell instance: 14.6 us as 68 chunks of eight, 5.3 as 538 of one).  Larger batches go
+// through the counter.
 template <int kMode, int kItems, bool kSeed>
-void launch_items(const oppb_advec_batch* b, oppb_move_status* status, int32_t max_hops, cudaStream_t s) {
-    const int grid = persistent_grid<kMode, kItems, kSeed>(ceil_div(b->n_work, kChunkItems));
-    advec_kernel<kMode, kItems, kSeed><<<grid, kAdvBlock, 0, s>>>(*b, status, max_hops);
+int launch_items(const oppb_advec_batch* b, oppb_move_status* status, int32_t max_hops, cudaStream_t s) {
+    const int resident = resident_blocks<kMode, kItems, kSeed>();
+    const int passes = ceil_div(b->n_work, kItems);
+    if (passes <= resident) {
+        advec_kernel<kMode, kItems, kSeed, true><<<passes, kAdvBlock, 0, s>>>(*b, status, max_hops, kItems);
+        return OPPB_OK;
+    }
+    if (cudaMemsetAsync(b->work_counter, 0, sizeof(int32_t), s) != cudaSuccess) return OPPB_ERR_LAUNCH;
+    const int chunks = ceil_div(b->n_work, kChunkItems);
+    const int grid = resident > 0 && resident < chunks ? resident : chunks;
+    advec_kernel<kMode, kItems, kSeed, false><<<grid, kAdvBlock, 0, s>>>(*b, status, max_hops, kChunkItems);
+    return OPPB_OK;
 }
 
 template <int kMode, bool kSeed>
-void launch_seeded(const oppb_advec_batch* b, oppb_move_status* status, int32_t max_hops, cudaStream_t s) {
+int launch_seeded(const oppb_advec_batch* b, oppb_move_status* status, int32_t max_hops, cudaStream_t s) {
     const int items = tuning().advec_items;
-    if (items == 4)
-        launch_items<kMode, 4, kSeed>(b, status, max_hops, s);
-    else if (items == 1)
-        launch_items<kMode, 1, kSeed>(b, status, max_hops, s);
-    else
-        launch_items<kMode, 2, kSeed>(b, status, max_hops, s);
+    // One item a block while every item has a resident block.
+    if (items == 1 || b->n_work <= resident_blocks<kMode, 1, kSeed>())
+        return launch_items<kMode, 1, kSeed>(b, status, max_hops, s);
+    return items == 4 ? launch_items<kMode, 4, kSeed>(b, status, max_hops, s)
+                      : launch_items<kMode, 2, kSeed>(b, status, max_hops, s);
 }
 
 // The pointers a launch reads or writes must be set: pos always, vel unless the launch only
@@ -390,15 +427,13 @@ int launch_advec(const oppb_advec_batch* b, oppb_move_status* status, int32_t ma
     if (kMode != kUpdateOnly && (!status || max_hops <= 0)) return OPPB_ERR_ARG;
     if (b->n_work == 0) return OPPB_OK;
     cudaStream_t s = as_stream(stream);
-    if (cudaMemsetAsync(b->work_counter, 0, sizeof(int32_t), s) != cudaSuccess) return OPPB_ERR_LAUNCH;
-    if constexpr (kMode != kUpdateOnly) {
-        if (b->dh)
-            launch_seeded<kMode, true>(b, status, max_hops, s);
-        else
-            launch_seeded<kMode, false>(b, status, max_hops, s);
-    } else {
-        launch_seeded<kMode, false>(b, status, max_hops, s);
-    }
+    int rc2 = OPPB_OK;
+    if constexpr (kMode != kUpdateOnly)
+        rc2 = b->dh ? launch_seeded<kMode, true>(b, status, max_hops, s)
+                    : launch_seeded<kMode, false>(b, status, max_hops, s);
+    else
+        rc2 = launch_seeded<kMode, false>(b, status, max_hops, s);
+    if (rc2) return rc2;
     count_launches(1);
     return launch_status();
 }
