@@ -7,9 +7,9 @@
 // kept pairs are a prefix: exactly the pairs of the reference's sequential loop
 // (opp_lib/src/core/opp_particle_organize_core.cpp:124-218).
 //   1. per-block hole counts over the bitmap,
-//   2. exclusive scan of the block counts,
-//   3. emit hole[k] and mover[k] for k < remove_count (ranks from the scan),
-//   4. copy every dat element mover[k] -> hole[k] for the kept pairs.
+//   2. emit hole[k] and mover[k] for k < remove_count (ranks from the counts, which every block
+//      sums itself up to kHfDirectBlocks blocks, else from an exclusive scan of them),
+//   3. copy every dat element mover[k] -> hole[k] for the kept pairs.
 
 #include <climits>
 #include <mutex>
@@ -21,8 +21,6 @@ namespace oppb {
 namespace {
 
 constexpr int kHfBlock = 256;
-// Two bitmap words (64 particles) a thread: the threads over the last live particles emit the
-// movers bit by bit, so this bounds the longest thread of the emit kernel.
 constexpr int kHfWordsPerThread = 2;
 constexpr int kHfWords = kHfBlock * kHfWordsPerThread;  // words per block (16,384 particles)
 constexpr int kMaxDats = 16;
@@ -75,62 +73,91 @@ __global__ void __launch_bounds__(kHfBlock) hf_count_kernel(const uint32_t* __re
     if (threadIdx.x == 0) block_holes[blockIdx.x] = total;
 }
 
-// block_base: exclusive hole prefix per block, block_base[n_blocks] = total holes H.
+// Emits the pairs' two sides.  block_holes: with kScanned the exclusive hole prefix per block and,
+// at [n_blocks], the total H; else the blocks' hole counts, which every block sums up to itself
+// (and to H): up to kHfDirectBlocks blocks that costs less than the scan's launch.  *total_out
+// receives H for the copy kernel.
+//
+// Latency-bound: thousands of threads do nothing but the few over the holes and the last live
+// particles, so what counts is the longest thread.  After the block's scan the words' prefixes go
+// through shared memory and each thread takes single bytes: at most eight particles one after
+// the other instead of 64 (460k particles, 2,000 removals: 4.4 us instead of 6.0).
+template <bool kScanned>
 __global__ void __launch_bounds__(kHfBlock) hf_emit_kernel(const uint32_t* __restrict__ bits, CountArg size_arg,
-                                                           int64_t n_words, const int* __restrict__ block_base,
+                                                           int64_t n_words, const int* __restrict__ block_holes,
                                                            int n_blocks, CountArg remove_arg,
                                                            int32_t* __restrict__ hole_list,
-                                                           int32_t* __restrict__ mover_list) {
+                                                           int32_t* __restrict__ mover_list, int* total_out) {
     __shared__ int sm[kHfBlock / 32 + 1];
+    __shared__ uint32_t s_word[kHfWords];
+    __shared__ int s_before[kHfWords];  // holes of the set before the word
     const int32_t size = resolve(size_arg);
     const int32_t remove_count = resolve(remove_arg);
-    // Thread t owns words [w0 + t*8, w0 + t*8 + 8) (blocked, so ranks follow index order).
-    const int64_t wt = (int64_t)blockIdx.x * kHfWords + (int64_t)threadIdx.x * kHfWordsPerThread;
+    int base, H;
+    if (kScanned) {
+        base = block_holes[blockIdx.x];
+        H = block_holes[n_blocks];
+    } else {
+        int before = 0, all = 0;
+        for (int b = threadIdx.x; b < n_blocks; b += kHfBlock) {
+            const int c = block_holes[b];
+            all += c;
+            before += b < (int)blockIdx.x ? c : 0;
+        }
+        block_exclusive_scan(before, sm, &base);
+        block_exclusive_scan(all, sm, &H);
+        if (blockIdx.x == 0 && threadIdx.x == 0) *total_out = H;
+    }
+    // Thread t owns kHfWordsPerThread consecutive words (blocked, so ranks follow index order).
+    const int64_t w0 = (int64_t)blockIdx.x * kHfWords;
+    const int t0 = threadIdx.x * kHfWordsPerThread;
     uint32_t w[kHfWordsPerThread];
     int c = 0;
 #pragma unroll
     for (int k = 0; k < kHfWordsPerThread; k++) {
-        w[k] = (wt + k < n_words) ? hole_word(bits, wt + k, size) : 0u;
+        w[k] = (w0 + t0 + k < n_words) ? hole_word(bits, w0 + t0 + k, size) : 0u;
         c += __popc(w[k]);
     }
     int total;
-    int holes_before = block_exclusive_scan(c, sm, &total) + block_base[blockIdx.x];
-    const int64_t H = block_base[n_blocks];
+    int before = block_exclusive_scan(c, sm, &total) + base;
+    // No pair lies in this block: no hole, and its last particle is not among the last
+    // remove_count live ones (live particles behind the block: all behind it less its holes).
     const int64_t live_total = (int64_t)size - H;
-#pragma unroll 1
+    const int64_t first0 = w0 * 32;
+    const int64_t behind = first0 + (int64_t)kHfWords * 32 < size ? size - (first0 + (int64_t)kHfWords * 32) : 0;
+    const int64_t live_behind = behind - ((int64_t)H - base - total);
+    if ((total == 0 || base >= remove_count) && live_behind >= remove_count) return;
+#pragma unroll
     for (int k = 0; k < kHfWordsPerThread; k++) {
-        const int64_t word = wt + k;
-        const int64_t first = word * 32;
-        if (first >= size) break;
-        const int n_valid = (size - first) < 32 ? (int)(size - first) : 32;
-        uint32_t hw = w[k];
-        // Holes: ascending rank holes_before, holes_before+1, ...
-        if (holes_before < remove_count) {
-            uint32_t m = hw;
-            int h = holes_before;
-            while (m && h < remove_count) {
-                const int b = __ffs(m) - 1;
-                m &= m - 1;
-                hole_list[h++] = (int32_t)(first + b);
+        s_word[t0 + k] = w[k];
+        s_before[t0 + k] = before;
+        before += __popc(w[k]);
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int e = threadIdx.x; e < kHfWords * 4; e += kHfBlock) {
+        const uint32_t word = s_word[e >> 2];
+        const int shift = (e & 3) * 8;
+        const int64_t first = first0 + (int64_t)(e >> 2) * 32 + shift;
+        if (first >= size) continue;
+        const uint32_t valid = size - first < 8 ? (1u << (int)(size - first)) - 1u : 0xffu;
+        const int holes_before = s_before[e >> 2] + __popc(word & ((1u << shift) - 1u));
+        uint32_t hb = (word >> shift) & valid;
+        uint32_t lb = ~(word >> shift) & valid;
+        // Holes: ascending rank.
+        for (int h = holes_before; hb && h < remove_count; h++) {
+            hole_list[h] = (int32_t)(first + (__ffs(hb) - 1));
+            hb &= hb - 1;
+        }
+        // Live particles: back rank = live_total - 1 - front rank, front rank = index - holes
+        // before it; the byte's last one has the smallest.
+        int64_t back = live_total - 1 - (first - holes_before);
+        if (back - __popc(lb) + 1 < remove_count) {
+            for (; lb; back--) {
+                if (back < remove_count) mover_list[back] = (int32_t)(first + (__ffs(lb) - 1));
+                lb &= lb - 1;
             }
         }
-        // Live particles: back rank = live_total - 1 - (index - holes before index).
-        // The largest live index of this word has the smallest back rank.
-        const int64_t live_first_rank = first - holes_before;  // front rank of first live in word
-        const int n_live = n_valid - __popc(hw);
-        if (n_live > 0) {
-            const int64_t min_back = live_total - 1 - (live_first_rank + n_live - 1);
-            if (min_back < remove_count) {
-                int64_t front = live_first_rank;
-                for (int b = 0; b < n_valid; b++) {
-                    if (hw & (1u << b)) continue;
-                    const int64_t back = live_total - 1 - front;
-                    if (back < remove_count) mover_list[back] = (int32_t)(first + b);
-                    front++;
-                }
-            }
-        }
-        holes_before += __popc(hw);
     }
 }
 
@@ -202,6 +229,34 @@ __global__ void __launch_bounds__(256) removal_bits_kernel(const int32_t* __rest
     if ((threadIdx.x & 31) == 0 && i < size) bits[i >> 5] = w;
 }
 
+// Blocks up to which the emit kernel sums the blocks' counts itself instead of a scan launch (4.2 us
+// and a gap): 16 loads a thread at the limit, 67M particles.  A captured ten-step cycle of 460k
+// particles takes 714 us instead of 796, a step-by-step one 525 instead of 540 (four steps).
+constexpr int kHfDirectBlocks = 4096;
+
+// The hole fill's launches.  block_holes: n_blocks + 1 ints.
+int launch_hole_fill(const uint32_t* remove_bits, const CountArg& sz, const CountArg& rc, int64_t n_words, int n_blocks,
+                     int* block_holes, int32_t* hole_list, int32_t* mover_list, int32_t stride, const DatList& dl,
+                     int copy_grid, cudaStream_t s) {
+    int* total = block_holes + n_blocks;
+    hf_count_kernel<<<n_blocks, kHfBlock, 0, s>>>(remove_bits, sz, n_words, block_holes);
+    if (n_blocks <= kHfDirectBlocks) {
+        hf_emit_kernel<false><<<n_blocks, kHfBlock, 0, s>>>(remove_bits, sz, n_words, block_holes, n_blocks, rc,
+                                                            hole_list, mover_list, total);
+    } else {
+        scan_single_block_kernel<<<1, kScanBlock, 0, s>>>(block_holes, n_blocks);
+        hf_emit_kernel<true><<<n_blocks, kHfBlock, 0, s>>>(remove_bits, sz, n_words, block_holes, n_blocks, rc,
+                                                           hole_list, mover_list, total);
+        count_launches(1);
+    }
+    count_launches(2);
+    if (dl.total_cols > 0) {
+        hf_copy_kernel<<<copy_grid, 256, 0, s>>>(rc, hole_list, mover_list, total, sz, stride, dl);
+        count_launches(1);
+    }
+    return launch_status();
+}
+
 size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
 }  // namespace
@@ -257,20 +312,8 @@ extern "C" int oppb_hole_fill(int32_t size, int32_t remove_count, const uint32_t
     int32_t* mover_list = reinterpret_cast<int32_t*>(ws);
 
     const CountArg sz{size, nullptr, 0}, rc{remove_count, nullptr, 0};
-    hf_count_kernel<<<n_blocks, kHfBlock, 0, s>>>(remove_bits, sz, n_words, block_base);
-    // block_base[0..n_blocks) exclusive, block_base[n_blocks] = total holes.
-    scan_single_block_kernel<<<1, kScanBlock, 0, s>>>(block_base, n_blocks);
-    (void)scan_tmp;
-    hf_emit_kernel<<<n_blocks, kHfBlock, 0, s>>>(remove_bits, sz, n_words, block_base, n_blocks, rc, hole_list,
-                                                 mover_list);
-    count_launches(3);
-    if (dl.total_cols > 0) {
-        const int64_t threads = (int64_t)remove_count * dl.total_cols;
-        hf_copy_kernel<<<ceil_div(threads, 256), 256, 0, s>>>(rc, hole_list, mover_list, block_base + n_blocks, sz,
-                                                             stride, dl);
-        count_launches(1);
-    }
-    return launch_status();
+    return launch_hole_fill(remove_bits, sz, rc, n_words, n_blocks, block_base, hole_list, mover_list, stride, dl,
+                            ceil_div((int64_t)remove_count * dl.total_cols, 256), s);
 }
 
 extern "C" size_t oppb_hole_fill_dev_workspace_bytes(int32_t size_bound) {
@@ -312,18 +355,9 @@ extern "C" int oppb_hole_fill_dev(int32_t size_bound, const oppb_set_count* coun
     // size_bound pairs, and no more than the count can be removed.
     const CountArg sz{size_bound, &count->size, pending};
     const CountArg rc{size_bound, &status->remove_count, 0};
-    hf_count_kernel<<<n_blocks, kHfBlock, 0, s>>>(remove_bits, sz, n_words, block_base);
-    scan_single_block_kernel<<<1, kScanBlock, 0, s>>>(block_base, n_blocks);
-    hf_emit_kernel<<<n_blocks, kHfBlock, 0, s>>>(remove_bits, sz, n_words, block_base, n_blocks, rc, hole_list,
-                                                 mover_list);
-    count_launches(3);
-    if (dl.total_cols > 0) {
-        const int64_t items = (int64_t)size_bound * dl.total_cols;
-        const int grid = ceil_div(items, 256) < 148 * 16 ? ceil_div(items, 256) : 148 * 16;
-        hf_copy_kernel<<<grid, 256, 0, s>>>(rc, hole_list, mover_list, block_base + n_blocks, sz, stride, dl);
-        count_launches(1);
-    }
-    return launch_status();
+    const int64_t copy_blocks = ceil_div((int64_t)size_bound * dl.total_cols, 256);
+    return launch_hole_fill(remove_bits, sz, rc, n_words, n_blocks, block_base, hole_list, mover_list, stride, dl,
+                            (int)(copy_blocks < 148 * 16 ? copy_blocks : 148 * 16), s);
 }
 
 extern "C" int oppb_step_end_dev(oppb_set_count* count, int32_t pending, const oppb_move_status* status,
@@ -433,16 +467,6 @@ extern "C" int oppb_hole_fill_static(int32_t size, int32_t remove_count, const u
     int32_t* mover_list = hole_list + kStaticListWords;
 
     const CountArg sz{size, nullptr, 0}, rc{remove_count, nullptr, 0};
-    hf_count_kernel<<<n_blocks, kHfBlock, 0, s>>>(remove_bits, sz, n_words, block_base);
-    scan_single_block_kernel<<<1, kScanBlock, 0, s>>>(block_base, n_blocks);
-    hf_emit_kernel<<<n_blocks, kHfBlock, 0, s>>>(remove_bits, sz, n_words, block_base, n_blocks, rc, hole_list,
-                                                 mover_list);
-    count_launches(3);
-    if (dl.total_cols > 0) {
-        const int64_t threads = (int64_t)remove_count * dl.total_cols;
-        hf_copy_kernel<<<ceil_div(threads, 256), 256, 0, s>>>(rc, hole_list, mover_list, block_base + n_blocks, sz,
-                                                             stride, dl);
-        count_launches(1);
-    }
-    return launch_status();
+    return launch_hole_fill(remove_bits, sz, rc, n_words, n_blocks, block_base, hole_list, mover_list, stride, dl,
+                            ceil_div((int64_t)remove_count * dl.total_cols, 256), s);
 }
