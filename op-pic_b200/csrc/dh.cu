@@ -80,8 +80,7 @@ struct TetCells {
     }
     __device__ bool holds(int32_t c, const double p[3]) const {
         double l[4];
-        int nb[4];
-        visit_f64(m, c, p[0], p[1], p[2], l, nb);
+        visit_f64(m, c, p[0], p[1], p[2], l);
         return inside_f64(l);
     }
 };

@@ -3,9 +3,9 @@
 //
 // One thread per particle; particles in SoA (stride = capacity).  A cell visit is a
 // dependent gather of the cell's record with 256-bit loads through the read-only path:
-// FP64 = 4 loads of the 128-B det record + 1 of the 32-B nav record {coef, c2c}; mixed =
-// 2 loads of the 64-B f32 record {3 lambda rows, origin}, + the 16-B c2c on a hop.  Lanes
-// of a warp share cells only while the particles are still close to their sorted order,
+// FP64 = 4 loads of the 128-B det record + the 8-B coefficient of the nav record {coef, c2c},
+// and 4 B of its neighbours on a hop; mixed = 2 loads of the 64-B f32 record {3 lambda rows,
+// origin} + 4 B of the c2c on a hop.  Lanes of a warp share cells only while the particles are still close to their sorted order,
 // so a load instruction pays up to one L1 sector per lane; the L1 data pipe is what
 // bounds the kernel, hence few wide loads per visit and a 32-register cap (full
 // occupancy hides the dependent-gather latency).
@@ -113,8 +113,7 @@ __device__ __forceinline__ double* deposit_target(const DepositArgs& d, int32_t 
 // would raise the register count of the whole kernel.
 __device__ __noinline__ void recheck_f64(const oppb_tet_mesh& m, int32_t c, double x, double y, double z,
                                          double* l) {
-    int nb[4];
-    visit_f64(m, c, x, y, z, l, nb);
+    visit_f64(m, c, x, y, z, l);
 }
 
 // Bookkeeping shared by all move variants: the warp's removal bitmap word, then the CTA's
@@ -386,11 +385,10 @@ __global__ void __launch_bounds__(kBlock, kThreadsPerSm / kBlock)
                 err = OPPB_ERR_CELL_RANGE;
                 break;
             }
-            int nb[4];
-            visit_f64(m, cell, x, y, z, l, nb);
+            visit_f64(m, cell, x, y, z, l);
             visits++;
             if (inside_f64(l)) break;
-            const int32_t next = pick(nb, argmin4(l));
+            const int32_t next = neighbour(m, cell, argmin4(l));
             if (next < 0) {
                 cell = kRemoved;
                 status = kNeedRemove;
@@ -969,8 +967,7 @@ __global__ void __launch_bounds__(kMoveBlock, kOcc)
             }
         }
         if (visits > 0) {  // the FP64 lambdas of the last cell visited, as move_f64_kernel leaves them
-            int nb[4];
-            visit_f64(m, last, x, y, z, l, nb);
+            visit_f64(m, last, x, y, z, l);
         }
         if (err) {
             raise_error(st, err, (int32_t)i);

@@ -21,30 +21,24 @@ __device__ __forceinline__ void swap_if(bool p, double& a, double& b) {
 }
 
 // lambda_0..3 of point (x,y,z) in cell c, evaluated exactly as the FP64 reference.
-// Also returns the cell's neighbours (nav record).
 //
 // The j-th 256-bit load of a lane reads sector j ^ (lane & 3) of its 128-B det record, so the
 // four lanes that a wide load serves together read four different sectors.  Lanes in different
 // cells that read the same sector index of their records hit the same L1 banks and are served
 // one after the other; with the sectors spread the fused FP64 move of the 57M-particle state
 // takes 3.46 ms instead of 4.39.  Each sector holds one vertex's four coefficients, so only the
-// four lambdas have to be put back in vertex order.
+// four lambdas have to be put back in vertex order.  Of the nav record a visit reads only the 8
+// bytes of the coefficient, a wavefront or two instead of the eight that a 256-bit load returns to
+// a warp at least; a particle that hops on reads its one neighbour (neighbour()): 3.46 -> 3.21 ms.
 __device__ __forceinline__ void visit_f64(const oppb_tet_mesh& m, int32_t c, double x, double y, double z,
-                                          double l[4], int nb[4]) {
+                                          double l[4]) {
     const double* d = m.det + (int64_t)c * 16;
     const uint32_t first = threadIdx.x & 3u;
     double r[16];
 #pragma unroll
     for (uint32_t j = 0; j < 4; j++)
         ldg256(d + ((j ^ first) << 2), r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
-    double coef, n01, n23, unused;
-    ldg256(m.nav + (int64_t)c * 4, coef, n01, n23, unused);
-    (void)unused;
-    const long long a = __double_as_longlong(n01), b = __double_as_longlong(n23);
-    nb[0] = (int)(a & 0xffffffffll);
-    nb[1] = (int)(a >> 32);
-    nb[2] = (int)(b & 0xffffffffll);
-    nb[3] = (int)(b >> 32);
+    const double coef = __ldg(m.nav + (int64_t)c * 4);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         double t = __dsub_rn(r[4 * i], __dmul_rn(r[4 * i + 1], x));
@@ -78,8 +72,9 @@ __device__ __forceinline__ int argmin4(const double l[4]) {
     return mi;
 }
 
-__device__ __forceinline__ int pick(const int nb[4], int i) {
-    return i == 0 ? nb[0] : i == 1 ? nb[1] : i == 2 ? nb[2] : nb[3];
+// The cell behind face i of cell c (the nav record's c2c), -1 at the boundary.
+__device__ __forceinline__ int32_t neighbour(const oppb_tet_mesh& m, int32_t c, int i) {
+    return __ldg(reinterpret_cast<const int32_t*>(m.nav + (int64_t)c * 4 + 1) + i);
 }
 
 }  // namespace
