@@ -8,7 +8,7 @@
 // are ordered by cell over the whole block (warp match, then a small hash table of the block's
 // cells), so that a thread sums one accumulator over a run of rows and issues one FP64 atomic per
 // cell of its run.  Bound by instruction issue and FP64 latency (the correctly rounded divides and
-// square roots).  104.9M particles of the two-stream state: 6.66 ms a call against 8.72 with the
+// square roots).  104.9M particles of the two-stream state: 5.76 ms a call against 8.72 with the
 // walk in place, one staged reduction a warp and the visit counters added once a warp.
 //
 // FP64 expressions are written in the reference's order and this file is compiled with
@@ -21,8 +21,10 @@
 namespace oppb {
 namespace {
 
-constexpr int kCabBlock = 256;
-constexpr int kCabWarps = kCabBlock / 32;
+// 128 threads, eight blocks an SM: a warp waits for three others at the block's barriers, not for
+// seven (256 threads: 6.49 ms on the two-stream state, 64: 6.66, 128: 6.01 with eight sum chunks).
+constexpr int kCabBlockBits = 7;
+constexpr int kCabBlock = 1 << kCabBlockBits;
 constexpr int kSparseLanes = 4;  // at most this many depositing lanes: plain atomics, no staging
 constexpr int kStageStride = 14;  // doubles per staged row: 12 used, 16-B aligned rows
 
@@ -323,54 +325,41 @@ struct CabShared {
     double rows[kCabBlock + 32][kStageStride];
     int32_t row_key[kCabBlock + 32];  // the cell of every row
     int32_t tab_key[kCabBlock];       // open-addressing table of the block's cells, -1 = free
-    int32_t tab_cnt[kCabBlock];       // rows of each, then the first row of each
-    int32_t warp_rows[kCabWarps];
+    int32_t tab_cnt[kCabBlock];       // rows of each
+    int32_t tab_first[kCabBlock];     // first row of each
+    int32_t n_rows;
     int32_t n_cross;
     uint16_t cross_row[kCabBlock];    // crossing particles: their row and their thread
     uint16_t cross_thread[kCabBlock];
 };
 
 // The row of this thread's values such that the rows of one cell are contiguous: lanes of a
-// warp with the same key take their place in the key's table slot together.  key < 0: no row.
-// Sets *n_rows to the block's row count.  Every thread of the block must call it.
-__device__ __forceinline__ int cell_ordered_row(CabShared& sh, int32_t key, int* n_rows) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// warp with the same key take their place in the key's table slot together, and the lane that
+// inserted a key takes the key's run of rows.  key < 0: no row.  sh.n_rows is the block's row count
+// afterwards.  Every thread of the block must call it.
+__device__ __forceinline__ int cell_ordered_row(CabShared& sh, int32_t key) {
+    const int lane = threadIdx.x & 31;
     const unsigned peers = __match_any_sync(kFullMask, key);
     const int leader = __ffs(peers) - 1;
     unsigned h = 0;
     int base = 0;
+    bool inserted = false;
     if (lane == leader && key >= 0) {
-        h = ((uint32_t)key * 2654435761u) >> 24;
+        h = ((uint32_t)key * 2654435761u) >> (32 - kCabBlockBits);
         for (int probe = 0; probe < kCabBlock; probe++) {  // at most kCabBlock distinct keys: one is free
             const int32_t k = atomicCAS(&sh.tab_key[h], -1, key);
-            if (k == -1 || k == key) break;
+            inserted = k == -1;
+            if (inserted || k == key) break;
             h = (h + 1) & (kCabBlock - 1);
         }
         base = atomicAdd(&sh.tab_cnt[h], __popc(peers));
     }
+    __syncthreads();
+    if (inserted) sh.tab_first[h] = atomicAdd(&sh.n_rows, sh.tab_cnt[h]);
     h = __shfl_sync(kFullMask, h, leader);
     base = __shfl_sync(kFullMask, base, leader);
     __syncthreads();
-    int incl = sh.tab_cnt[threadIdx.x];
-    const int own = incl;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(kFullMask, incl, o);
-        if (lane >= o) incl += v;
-    }
-    if (lane == 31) sh.warp_rows[warp] = incl;
-    __syncthreads();
-    int first = incl - own, total = 0;
-#pragma unroll
-    for (int w = 0; w < kCabWarps; w++) {
-        const int c = sh.warp_rows[w];
-        first += w < warp ? c : 0;
-        total += c;
-    }
-    sh.tab_cnt[threadIdx.x] = first;
-    __syncthreads();
-    *n_rows = total;
-    return sh.tab_cnt[h] + base + __popc(peers & lanemask_lt());
+    return sh.tab_first[h] + base + __popc(peers & lanemask_lt());
 }
 
 __device__ __forceinline__ void write_row(double* row, const double* j) {
@@ -385,14 +374,17 @@ __device__ __forceinline__ int32_t through_face(const HexArgs& m, int32_t cell, 
     return (uint32_t)next < (uint32_t)m.n_cells ? next : -1;
 }
 
-constexpr int kSumChunks = 10;                     // row ranges of the block's sums
+// Row ranges of the block's sums: fewer ranges mean fewer atomics and more steps a thread (two-stream
+// state: 6.01, 5.97, 5.76, 5.96 ms for 8, 6, 5, 4; five ranges fill two warps).
+constexpr int kSumChunks = 5;
 constexpr int kSumThreads = kSumChunks * 12;       // one thread per range and accumulator
 static_assert(kSumThreads <= kCabBlock - 32, "the sums fit beside the crossing particles' warp");
 
-// kOcc: resident CTAs per SM the kernel is compiled for (oppb_tuning.cabana_occupancy): 0 = the
-// compiler's register count, 4 (64 registers) or 5 (48 registers).
+// kOcc: resident warps per SM the kernel is compiled for in units of eight, the CTAs of 256 threads
+// that oppb_tuning.cabana_occupancy counts: 0 = the compiler's register count, 4 (64 registers) or
+// 5 (48 registers).
 template <bool kF32Mom, int kOcc>
-__global__ void __launch_bounds__(kCabBlock, kOcc > 0 ? kOcc : 1) cabana_move_deposit_kernel(HexArgs m, CabParts p,
+__global__ void __launch_bounds__(kCabBlock, kOcc > 0 ? kOcc * 256 / kCabBlock : 1) cabana_move_deposit_kernel(HexArgs m, CabParts p,
                                                                         oppb_cabana_consts k, ConstsF32 kf,
                                                                         double* acc, int32_t acc_stride,
                                                                         oppb_move_status* st, int32_t max_hops) {
@@ -404,7 +396,7 @@ __global__ void __launch_bounds__(kCabBlock, kOcc > 0 ? kOcc : 1) cabana_move_de
     const int64_t sd = p.stride;
     sh.tab_key[threadIdx.x] = -1;
     sh.tab_cnt[threadIdx.x] = 0;
-    if (threadIdx.x == 0) sh.n_cross = 0;
+    if (threadIdx.x == 0) sh.n_rows = sh.n_cross = 0;
     const bool active = i < p.size;
     const int32_t cell = active ? ld_stream(p.p2c + i) : -1;
     const bool pushed = active && (uint32_t)cell < (uint32_t)m.n_cells;
@@ -424,8 +416,8 @@ __global__ void __launch_bounds__(kCabBlock, kOcc > 0 ? kOcc : 1) cabana_move_de
         q = __ldg(p.weight + i) * k.qsp;
     }
     __syncthreads();
-    int n_rows;
-    int row = cell_ordered_row(sh, pushed ? cell : -1, &n_rows);
+    int row = cell_ordered_row(sh, pushed ? cell : -1);
+    const int n_rows = sh.n_rows;
 
     // The push (OPP_DO_ONCE).  A particle that stays in its cell is finished; one that leaves it
     // queues, with its state in its row, for the streak walk by a full warp below.

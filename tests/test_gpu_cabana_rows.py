@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("precision", ["f64", "mixed"])
-@pytest.mark.parametrize("n", [1, 31, 255, 256, 257, 1030])
+@pytest.mark.parametrize("n", [1, 31, 127, 128, 129, 256, 1030])
 @pytest.mark.parametrize("cells,scale", [("each", 3.0), ("each", 0.0), ("one", 3.0), ("mixed", 0.3)])
 def test_rows_and_queue(n, cells, scale, precision):
     mesh = HexMesh(9, 8, 17)
