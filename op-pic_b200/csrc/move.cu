@@ -981,10 +981,62 @@ __global__ void __launch_bounds__(kMoveBlock, kOcc)
 
 // ------------------------------------------------------------- standalone deposit
 
+// One warp's weights ordered by cell, and per cell group its cell, first row and size.
+struct WarpRows {
+    double w[32][4];
+    int32_t key[32];
+    uint16_t span[32];  // first row | size << 8
+};
+
+// warp_deposit through shared memory: the lanes' weights go to rows in the order of their cell groups
+// (and of the lanes inside one), lane 4g + v sums weight v of group g and adds it to the group's
+// node v, eight groups a pass.  A warp takes as many steps as its largest group has members, one
+// load each, where the shuffle loop takes eight shuffles a step: 6.9M cell-sorted particles 73 us
+// instead of 166.  The fused kernels keep the shuffles: the rows come off the L1 cache their
+// walks live in (push + move + deposit of 57M particles: 3.51 against 3.47 ms).
+__device__ __forceinline__ void warp_deposit_rows(const oppb_tet_mesh& m, WarpRows& rows, double* target, int32_t key,
+                                                  const double l[4]) {
+    const int lane = threadIdx.x & 31;
+    const unsigned peers = __match_any_sync(kFullMask, key);
+    const int leader = __ffs(peers) - 1;
+    const bool leads = key >= 0 && lane == leader;
+    const unsigned leaders = __ballot_sync(kFullMask, leads);
+    if (leaders == 0u) return;
+    const int size = leads ? __popc(peers) : 0;
+    int first = size;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(kFullMask, first, o);
+        if (lane >= o) first += v;
+    }
+    first = __shfl_sync(kFullMask, first - size, leader);
+    if (leads) {
+        const int g = __popc(leaders & lanemask_lt());
+        rows.key[g] = key;
+        rows.span[g] = (uint16_t)(first | (size << 8));
+    }
+    if (key >= 0) {
+        double2* w = reinterpret_cast<double2*>(rows.w[first + __popc(peers & lanemask_lt())]);
+        w[0] = make_double2(l[0], l[1]);
+        w[1] = make_double2(l[2], l[3]);
+    }
+    __syncwarp();
+    const int v = lane & 3, n_groups = __popc(leaders);
+    for (int g = lane >> 2; g < n_groups; g += 8) {
+        const int32_t node = __ldg(m.c2n + (int64_t)rows.key[g] * 4 + v);
+        const int span = rows.span[g], n = span >> 8;
+        const double* w = &rows.w[span & 31][v];
+        double sum = w[0];
+        for (int k = 1; k < n; k++) sum += w[4 * k];
+        if ((uint32_t)node < (uint32_t)m.n_nodes) atomicAdd(target + node, sum);
+    }
+}
+
 template <int kDep>
 __global__ void __launch_bounds__(kMoveBlock, kMinBlocks)
     deposit_f64_kernel(oppb_tet_mesh m, PartArgs p, DepositArgs dep) {
     __shared__ NodeTable table;
+    __shared__ __align__(16) WarpRows rows[kDep == kDepWarp ? kMoveBlock / 32 : 1];
     if (kDep == kDepTable) table_init(table);
     const int64_t i = (int64_t)blockIdx.x * kMoveBlock + threadIdx.x;
     const bool active = i < p.size;
@@ -997,7 +1049,10 @@ __global__ void __launch_bounds__(kMoveBlock, kMinBlocks)
         l[2] = ld_stream(p.lc + 2 * (int64_t)p.stride + i);
         l[3] = ld_stream(p.lc + 3 * (int64_t)p.stride + i);
     }
-    deposit_epilogue<kDep>(m, table, dep, ok, cell, l);
+    if constexpr (kDep == kDepWarp)
+        warp_deposit_rows(m, rows[threadIdx.x >> 5], deposit_target(dep, m.n_nodes), ok ? cell : -1, l);
+    else
+        deposit_epilogue<kDep>(m, table, dep, ok, cell, l);
 }
 
 // node_charge[n] += sum over copies r of copies[r][n].
