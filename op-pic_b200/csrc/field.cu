@@ -295,18 +295,18 @@ __global__ void __launch_bounds__(kFieldBlock) field_newton_kernel(FieldArgs a) 
 // Systems of up to kClusterNeq unknowns run as one thread-block cluster, whose barrier and
 // distributed shared memory replace the polled slots in global memory.  kCluster = false is a
 // cooperative launch of one block per SM.  At 458,591 unknowns (15 diagonals) an iteration takes
-// 14.6 us instead of 25.9 in field_newton_kernel, at 138,303 9.6 instead of 14.5.
+// 13.4 us instead of 25.9 in field_newton_kernel, at 138,303 8.0 instead of 14.5.  Of the 13.4 the
+// product takes 5 (K streamed from L2, then shared memory), the two reductions 6.
 
 constexpr int kCgMaxThreads = 640;  // 102 registers a thread
 constexpr int kCgMaxRows = 8;       // rows a thread
 constexpr int kCgMinRows = 64;      // rows a block, where there are as many
-constexpr int kStage = 8;           // window loads in flight a thread
+constexpr int kStage = 4;           // window loads in flight a thread
 constexpr int kCgMaxCluster = 16;
 constexpr int kCgMaxWarps = kCgMaxThreads / 32;
 constexpr int kCgMaxBlocks = 160;  // of the grid form
 
-constexpr int kCgSlots = (kCgMaxBlocks + 31) / 32;  // blocks' sums a lane of the polling warp reads
-constexpr int kCgMaxPolls = 1 << 20;                // about a second
+constexpr int kCgMaxPolls = 1 << 20;  // about a second
 
 // One block's sums in global memory: each value and the number of the reduction it belongs to are
 // one 16-byte word, so that a block that reads the number has the value too.  A slot fills a
@@ -323,7 +323,7 @@ struct __align__(128) CgSlot {
 
 __device__ __forceinline__ void post_word(CgWord* p, double v, unsigned long long turn) {
     const unsigned __int128 w = ((unsigned __int128)turn << 64) | (unsigned long long)__double_as_longlong(v);
-    asm volatile("st.release.gpu.global.b128 [%0], %1;" ::"l"(p), "q"(w) : "memory");
+    asm volatile("st.relaxed.gpu.global.b128 [%0], %1;" ::"l"(p), "q"(w) : "memory");
 }
 __device__ __forceinline__ bool poll_word(const CgWord* p, unsigned long long turn, double& v) {
     unsigned __int128 w;
@@ -332,11 +332,11 @@ __device__ __forceinline__ bool poll_word(const CgWord* p, unsigned long long tu
     return (unsigned long long)(w >> 64) == turn;
 }
 
-// Reduction scratch of a block.
+// Reduction scratch of a block, indexed [value].
 struct CgShared {
-    double2 part[2][kCgMaxCluster * kCgMaxWarps];  // cluster form: the sums of every warp of the cluster
-    double2 warp[kCgMaxWarps];                     // grid form: the block's warps
-    double2 sum;
+    double part[2][2][kCgMaxCluster * kCgMaxWarps];  // cluster form: the sums of every warp of the cluster
+    double warp[2][kCgMaxWarps];                     // grid form: the block's warps
+    double sum[2];
     int failed;
 };
 
@@ -348,83 +348,92 @@ struct CgArgs {
     CgSlot* slots;     // [2][gridDim.x], grid form; zeroed before the launch
 };
 
+// Sums over the lanes that hold one value: all 32 for kValues = 1, else lanes 0..15 hold the first
+// and 16..31 the second.
 template <int kValues>
-__device__ __forceinline__ void warp_sum(double2& v) {
+__device__ __forceinline__ double lane_sum(double v) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        v.x += __shfl_xor_sync(kFullMask, v.x, o);
-        if (kValues == 2) v.y += __shfl_xor_sync(kFullMask, v.y, o);
-    }
+    for (int o = kValues == 2 ? 8 : 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFullMask, v, o);
+    return v;
 }
 
 // Sum of v (its first kValues doubles) over all threads of all blocks, the same bits in every
-// thread, and a barrier of all blocks: what any thread wrote before, every thread sees after.
-// turn counts the reductions of the launch from 1.
+// thread.  With kBarrier it is also a barrier of all blocks: what any thread wrote before, every
+// thread sees after.  turn counts the reductions of the launch from 1.
 //
-// Cluster form: every warp stores its sum into every block's shared memory, then one cluster
-// barrier.  Grid form: the block's sum goes to its slot together with the turn, and warp 0 polls
-// the slots of all blocks, so that the reduction and the barrier are one round trip through L2
-// (a cooperative-groups grid barrier with the partial sums beside it took 7 us).  The blocks
-// are all resident (cooperative launch); a wait that runs out sets sh.failed.
-template <int kValues, bool kCluster>
-__device__ __forceinline__ double2 cg_all_sum(double2 v, CgShared& sh, CgSlot* slots, unsigned turn) {
+// Two values travel as one: half the lanes reduce the first, half the second, which shortens the
+// chain of shuffles.  Cluster form: every warp stores its sums into every block's shared memory,
+// then one cluster barrier.  Grid form: the block's sums go to its slot together with the turn, and
+// warp 0 polls the slots of all blocks, so that the reduction and the barrier are one round trip
+// through L2 (a cooperative-groups grid barrier with the partial sums beside it took 7 us).  The
+// blocks are all resident (cooperative launch); a wait that runs out sets sh.failed.
+template <int kValues, bool kBarrier, bool kCluster>
+__device__ __forceinline__ double2 cg_all_sum(double2 in, CgShared& sh, CgSlot* slots, unsigned turn) {
+    constexpr int kLanes = 32 / kValues;  // lanes a value
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
+    const int sub = lane % kLanes, value = lane / kLanes;
     const int n_blocks = (int)gridDim.x;
-    warp_sum<kValues>(v);
-    if (kCluster) {
-        double2* mine = &sh.part[turn & 1][blockIdx.x * n_warps + warp];
-        if (lane < n_blocks) *cg::this_cluster().map_shared_rank(mine, lane) = v;
-        cg::this_cluster().sync();
-        v = make_double2(0.0, 0.0);
-        for (int w = lane; w < n_blocks * n_warps; w += 32) {
-            v.x += sh.part[turn & 1][w].x;
-            if (kValues == 2) v.y += sh.part[turn & 1][w].y;
-        }
-        warp_sum<kValues>(v);
-        return v;
+    double v = in.x;
+    if (kValues == 2) {
+        const double other = __shfl_xor_sync(kFullMask, value == 0 ? in.y : in.x, 16);
+        v = (value == 0 ? in.x : in.y) + other;
     }
-    if (lane == 0) sh.warp[warp] = v;
+    v = lane_sum<kValues>(v);
+    if (kCluster) {
+        double* mine = &sh.part[turn & 1][value][blockIdx.x * n_warps + warp];
+        if (sub < n_blocks) *cg::this_cluster().map_shared_rank(mine, sub) = v;
+        cg::this_cluster().sync();
+        double2 s = make_double2(0.0, 0.0);
+        for (int w = lane; w < n_blocks * n_warps; w += 32) {
+            s.x += sh.part[turn & 1][0][w];
+            if (kValues == 2) s.y += sh.part[turn & 1][1][w];
+        }
+        v = s.x;
+        if (kValues == 2) {
+            const double other = __shfl_xor_sync(kFullMask, value == 0 ? s.y : s.x, 16);
+            v = (value == 0 ? s.x : s.y) + other;
+        }
+        v = lane_sum<kValues>(v);
+        if (kValues == 1) return make_double2(v, 0.0);
+        return make_double2(__shfl_sync(kFullMask, v, 0), __shfl_sync(kFullMask, v, 16));
+    }
+    if (sub == 0) sh.warp[value][warp] = v;
     __syncthreads();
     if (warp == 0) {
-        v = lane < n_warps ? sh.warp[lane] : make_double2(0.0, 0.0);
-        warp_sum<kValues>(v);
+        v = 0.0;
+        for (int w = sub; w < n_warps; w += kLanes) v += sh.warp[value][w];
+        v = lane_sum<kValues>(v);
         CgSlot* at = slots + (turn & 1) * n_blocks;
-        if (lane == 0) {
-            __threadfence();
-            post_word(&at[blockIdx.x].value[0], v.x, turn);
-            if (kValues == 2) post_word(&at[blockIdx.x].value[1], v.y, turn);
+        if (sub == 0) {
+            if (kBarrier) __threadfence();
+            post_word(&at[blockIdx.x].value[value], v, turn);
         }
-        double x[kCgSlots], y[kCgSlots];
+        constexpr int kSlots = (kCgMaxBlocks + kLanes - 1) / kLanes;
+        double x[kSlots];
         bool all = false;
         for (int poll = 0; !all && poll < kCgMaxPolls; poll++) {
             bool here = true;
 #pragma unroll
-            for (int k = 0; k < kCgSlots; k++) {
-                const int b = lane + 32 * k;
-                x[k] = y[k] = 0.0;
+            for (int k = 0; k < kSlots; k++) {
+                const int b = sub + kLanes * k;
+                x[k] = 0.0;
                 if (b < n_blocks) {
-                    const bool first = poll_word(&at[b].value[0], turn, x[k]);
-                    const bool second = kValues == 1 || poll_word(&at[b].value[1], turn, y[k]);
-                    here = here && first && second;
+                    const bool posted = poll_word(&at[b].value[value], turn, x[k]);
+                    here = here && posted;
                 }
             }
             all = __all_sync(kFullMask, here);
         }
-        __threadfence();
-        v = make_double2(0.0, 0.0);
+        if (kBarrier) __threadfence();
+        v = 0.0;
 #pragma unroll
-        for (int k = 0; k < kCgSlots; k++) {
-            v.x += x[k];
-            if (kValues == 2) v.y += y[k];
-        }
-        warp_sum<kValues>(v);
-        if (lane == 0) {
-            sh.sum = v;
-            if (!all) sh.failed = 1;
-        }
+        for (int k = 0; k < kSlots; k++) v += x[k];
+        v = lane_sum<kValues>(v);
+        if (sub == 0) sh.sum[value] = v;
+        if (lane == 0 && !all) sh.failed = 1;
     }
     __syncthreads();
-    return sh.sum;
+    return make_double2(sh.sum[0], kValues == 2 ? sh.sum[1] : 0.0);
 }
 
 template <int kRows, bool kCluster>
@@ -438,21 +447,21 @@ __global__ void __launch_bounds__(kCgMaxThreads, 1) field_cg_kernel(const __grid
     double* pw = dyn;          // p of rows [r0 - lo, r0 + rows + hi)
     double* km = dyn + width;  // [smem_diag][rows]
     double* zg = a.q;          // z of all rows, the only vector blocks exchange
-    const int32_t stream_diag = a.n_diag - c.smem_diag;
     unsigned turn = 1;
     if (threadIdx.x == 0) sh.failed = 0;
     for (int32_t i = threadIdx.x; i < width; i += blockDim.x) pw[i] = 0.0;
+    const int32_t stream_diag = a.n_diag - c.smem_diag;
     for (int32_t j = 0; j < c.smem_diag; j++)
         for (int32_t i = threadIdx.x; i < n_own; i += blockDim.x)
             km[(int64_t)j * c.rows + i] = __ldg(a.dia_val + (int64_t)(stream_diag + j) * a.neq + r0 + i);
 
     // B = K D - F0 - F1, J's diagonal, z = r / diag (p starts as z).
-    double x[kRows], r[kRows], dg[kRows];
+    double x[kRows], r[kRows], dg[kRows], z[kRows];
     double2 v = make_double2(0.0, 0.0);
 #pragma unroll
     for (int k = 0; k < kRows; k++) {
         const int32_t i = threadIdx.x + k * blockDim.x;
-        x[k] = 0.0, r[k] = 0.0, dg[k] = 1.0;
+        x[k] = 0.0, r[k] = 0.0, dg[k] = 1.0, z[k] = 0.0;
         if (i >= n_own) continue;
         const int64_t u = r0 + i;
         double kd = 0.0, kuu = 0.0;
@@ -464,31 +473,43 @@ __global__ void __launch_bounds__(kCgMaxThreads, 1) field_cg_kernel(const __grid
         }
         r[k] = (kd - a.f0[u]) - a.f1[u];
         dg[k] = kuu + (-a.t2[u]);
-        const double z = r[k] / dg[k];
-        __stcg(zg + u, z);
-        v.x += r[k] * z;
+        z[k] = r[k] / dg[k];
+        __stcg(zg + u, z[k]);
+        v.x += r[k] * z[k];
         v.y += r[k] * r[k];
     }
-    v = cg_all_sum<2, kCluster>(v, sh, c.slots, turn++);
+    v = cg_all_sum<2, true, kCluster>(v, sh, c.slots, turn++);
     double rz = v.x, rr = v.y;
     const double b_norm = sqrt(rr);
     const double stop = fmax(a.rtol * b_norm, a.atol);
     double beta = 0.0;
     int it = 0;
     while (it < a.max_iter && sqrt(rr) > stop) {
-        // p = z + beta p over the window, kStage loads of z in flight a thread.
-        for (int32_t i0 = threadIdx.x; i0 < width; i0 += kStage * blockDim.x) {
-            double z[kStage];
+        // p = z + beta p over the window: the block's own rows from registers, the rest with kStage
+        // loads of z in flight a thread.
+        const int32_t halo = c.lo + c.hi;
+        for (int32_t i0 = threadIdx.x; i0 < halo; i0 += kStage * blockDim.x) {
+            double zw[kStage];
 #pragma unroll
             for (int k = 0; k < kStage; k++) {
-                const int32_t i = i0 + k * blockDim.x, u = r0 - c.lo + i;
-                z[k] = i < width && (uint32_t)u < (uint32_t)a.neq ? __ldcg(zg + u) : 0.0;
+                int32_t i = i0 + k * blockDim.x;
+                const bool in = i < halo;
+                if (i >= c.lo) i += c.rows;
+                const int32_t u = r0 - c.lo + i;
+                zw[k] = in && (uint32_t)u < (uint32_t)a.neq ? __ldcg(zg + u) : 0.0;
             }
 #pragma unroll
             for (int k = 0; k < kStage; k++) {
-                const int32_t i = i0 + k * blockDim.x;
-                if (i < width) pw[i] = z[k] + beta * pw[i];
+                int32_t i = i0 + k * blockDim.x;
+                const bool in = i < halo;
+                if (i >= c.lo) i += c.rows;
+                if (in) pw[i] = zw[k] + beta * pw[i];
             }
+        }
+#pragma unroll
+        for (int k = 0; k < kRows; k++) {
+            const int32_t i = threadIdx.x + k * blockDim.x;
+            if (i < n_own) pw[c.lo + i] = z[k] + beta * pw[c.lo + i];
         }
         __syncthreads();
         // The product, the diagonals in ascending order of their offset: each row's terms in
@@ -530,7 +551,7 @@ __global__ void __launch_bounds__(kCgMaxThreads, 1) field_cg_kernel(const __grid
             const int32_t i = threadIdx.x + k * blockDim.x;
             if (i < n_own) v.x += pw[i + c.lo] * s[k];
         }
-        v = cg_all_sum<1, kCluster>(v, sh, c.slots, turn++);
+        v = cg_all_sum<1, false, kCluster>(v, sh, c.slots, turn++);
         if (!kCluster && sh.failed) break;
         const double alpha = rz / v.x;
         v = make_double2(0.0, 0.0);
@@ -540,12 +561,12 @@ __global__ void __launch_bounds__(kCgMaxThreads, 1) field_cg_kernel(const __grid
             if (i >= n_own) continue;
             x[k] += alpha * pw[i + c.lo];
             r[k] = r[k] - alpha * s[k];
-            const double z = r[k] / dg[k];
-            __stcg(zg + r0 + i, z);
-            v.x += r[k] * z;
+            z[k] = r[k] / dg[k];
+            __stcg(zg + r0 + i, z[k]);
+            v.x += r[k] * z[k];
             v.y += r[k] * r[k];
         }
-        v = cg_all_sum<2, kCluster>(v, sh, c.slots, turn++);
+        v = cg_all_sum<2, true, kCluster>(v, sh, c.slots, turn++);
         if (!kCluster && sh.failed) break;
         beta = v.x / rz;
         rz = v.x;
@@ -650,9 +671,9 @@ struct CgPlan {
 };
 
 // Up to this many unknowns the CG runs as one cluster, above as one block per SM.  Microseconds an
-// iteration, cluster / grid: 4.2 / 7.3 at 4,719 unknowns, 6.1 / 7.9 at 18,207, 9.0 / 7.9 at 34,839
+// iteration, cluster / grid: 4.3 / 6.1 at 4,719 unknowns, 6.1 / 6.4 at 18,207, 9.0 / 6.3 at 34,839
 // (all in field_newton_kernel: 12.9, 13.7, 13.4).
-constexpr int kClusterNeq = 24576;
+constexpr int kClusterNeq = 18432;
 
 CgPlan cg_plan(int32_t neq, int32_t n_diag, int32_t lo, int32_t hi, int sms, int smem_max, bool cluster) {
     CgPlan p;

@@ -1,4 +1,4 @@
-"""The Newton step on K by diagonals (one cluster up to 24,576 unknowns, one block per SM above)
+"""The Newton step on K by diagonals (one cluster up to 18,432 unknowns, one block per SM above)
 against the same step on K as CSR, which the general kernel takes, around the edges of the split
 of rows over blocks and threads.  Both run the same CG on bit-identical products and differ in
 the order of the dot products and of the F1 / J-diagonal atomics only: the iteration counts agree
@@ -19,7 +19,7 @@ UNIT = dict(n0=1.0, phi0=0.0, kte=100.0, qe=1.0, eps0=1.0)
 
 # (nx, ny, nz): three 64-row blocks; 5 rows past 16 x 64; a wide window; the last mesh of the cluster
 # form and the first of the grid form; several rows a thread with K partly streamed.
-DIMS = [(4, 4, 8), (6, 6, 22), (40, 9, 12), (18, 18, 66), (20, 20, 64), (44, 44, 150)]
+DIMS = [(4, 4, 8), (6, 6, 22), (40, 9, 12), (16, 16, 64), (17, 17, 60), (44, 44, 150)]
 
 
 @pytest.mark.parametrize("dims", DIMS, ids=str)
