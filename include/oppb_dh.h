@@ -123,6 +123,30 @@ int oppb_move_ex(const oppb_tet_mesh* mesh, const oppb_particles* parts, const o
                  double* node_charge, oppb_move_status* status, int32_t max_hops, void* workspace,
                  size_t ws_bytes, void* stream);
 
+/* A host-sized FemPIC step up to its move, for oppb_step_begin. */
+typedef struct oppb_step {
+    const oppb_tet_mesh* mesh;
+    const oppb_inlet*    inlet;
+    const double*        rnd;             /* the injection table, as oppb_inject_f64            */
+    int32_t              rnd_stride, rnd_dim;
+    int32_t              n_inject;        /* the last n_inject particles of the set are injected */
+    int32_t              n_nodes;
+    double               ion_velocity;
+    oppb_move_options    move;            /* qm and dt are the injection's and the push's too    */
+    int32_t              separate_push;   /* 1: a push launch before the move (move.push = 0)    */
+    int32_t              max_hops;
+    double*              node_charge;     /* zeroed before the move                              */
+    oppb_move_status*    status;          /* device                                              */
+    oppb_move_status*    status_host;     /* page-locked host memory                             */
+    void*                workspace;       /* the deposit's                                       */
+    size_t               workspace_bytes;
+} oppb_step;
+
+/* oppb_inject_f64, the node charges' reset, the push when it is separate and oppb_move_ex in one
+ * call, then the status read into status_host; synchronises the stream, as the reference reads
+ * its remove count after the move.  parts->size counts the particles to inject. */
+int oppb_step_begin(const oppb_step* step, const oppb_particles* parts, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

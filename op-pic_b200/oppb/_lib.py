@@ -103,6 +103,8 @@ class DhGrid(C.Structure):
                 ("inv_spacing", C.c_double), ("dims", c_i64 * 3), ("size", c_i64), ("map", c_vp)]
 
 
+P = C.POINTER
+
 PRECISION_F64 = 0
 PRECISION_MIXED = 1
 
@@ -111,6 +113,13 @@ class MoveOptions(C.Structure):
     _fields_ = [("precision", c_i32), ("deposit", c_i32), ("push", c_i32), ("reserved", c_i32),
                 ("qm", C.c_double), ("dt", C.c_double), ("band", C.c_double), ("dh", C.POINTER(DhGrid)),
                 ("set_count", c_vp), ("pending", c_i32), ("reserved2", c_i32)]
+
+
+class Step(C.Structure):
+    _fields_ = [("mesh", P(TetMesh)), ("inlet", P(Inlet)), ("rnd", c_vp), ("rnd_stride", c_i32), ("rnd_dim", c_i32),
+                ("n_inject", c_i32), ("n_nodes", c_i32), ("ion_velocity", C.c_double), ("move", MoveOptions),
+                ("separate_push", c_i32), ("max_hops", c_i32), ("node_charge", c_vp), ("status", c_vp),
+                ("status_host", c_vp), ("workspace", c_vp), ("workspace_bytes", C.c_size_t)]
 
 
 class FieldSystem(C.Structure):
@@ -145,7 +154,6 @@ class FemPICMesh(C.Structure):
                 ("if_u", c_dp), ("if_v", c_dp), ("if_norm", c_dp), ("if_area", c_dp), ("if_n_pos", c_dp)]
 
 
-P = C.POINTER
 _SIGS = {
     "oppb_version": (C.c_char_p, []),
     "oppb_status_string": (C.c_char_p, [C.c_int]),
@@ -215,6 +223,7 @@ _SIGS = {
     "oppb_dh_build_quad": (C.c_int, [c_vp, c_i32, C.c_double, P(DhGrid), c_vp, C.c_size_t, P(C.c_size_t), c_vp]),
     "oppb_move_ex": (C.c_int, [P(TetMesh), P(Particles), P(MoveOptions), c_vp, c_vp, c_i32, c_vp, C.c_size_t,
                                c_vp]),
+    "oppb_step_begin": (C.c_int, [P(Step), P(Particles), c_vp]),
     "oppb_field_setup": (C.c_int, [P(FemPICMesh), P(FieldSystem)]),
     "oppb_field_system_free": (None, [P(FieldSystem)]),
     "oppb_field_work_doubles": (C.c_size_t, [c_i32]),

@@ -189,6 +189,7 @@ class ParticleSet:
         self.capacity = 0
         self.alloc_mult = alloc_mult
         self.status = torch.zeros(32 // 4, dtype=torch.int32, device=device)
+        self._dats = {}  # the dats' C structures by their buffers (two sets alternate through the sorts)
         self._alloc(capacity)
 
     def _alloc(self, cap: int) -> None:
@@ -202,6 +203,7 @@ class ParticleSet:
             setattr(self, name + "_swap", torch.empty_like(buf))
         self.bits = torch.zeros((max(cap, 1) + 31) // 32, dtype=torch.int32, device=self.device)
         self.capacity = cap
+        self._dats.clear()
 
     def increase(self, count: int) -> None:
         """opp_increase_particle_count_core semantics (capacity = size + count*alloc_mult),
@@ -215,6 +217,15 @@ class ParticleSet:
                            _ptr(self.bits))
 
     def dat_list(self):
+        key = tuple(_ptr(getattr(self, name)) for name, _, _ in self.DATS)
+        arr = self._dats.get(key)
+        if arr is None:
+            if len(self._dats) >= 2:
+                self._dats.clear()
+            arr = self._dats[key] = self._dat_structs()
+        return arr
+
+    def _dat_structs(self):
         arr = (L.Dat * len(self.DATS))()
         for k, (name, dim, dt) in enumerate(self.DATS):
             arr[k] = L.Dat(_ptr(getattr(self, name)), _ptr(getattr(self, name + "_swap")), dim,
@@ -290,6 +301,10 @@ class FemPIC:
         self._ws = torch.empty(0, dtype=torch.uint8, device=self.device)
         self._dep_ws = torch.empty(0, dtype=torch.uint8, device=self.device)
         self.lib = L.load()
+        # step()'s arguments of oppb_step_begin and the page-locked status it reads the move's into
+        self._status_pinned = torch.zeros(32 // 4, dtype=torch.int32).pin_memory()
+        self._status_host = L.MoveStatus.from_address(self._status_pinned.data_ptr())
+        self._step_args = L.Step()
         self.last = {}
         self._pipe = None  # run_steps' copy stream, events and double buffers, made once
         # Global move: every walk starts from the cell of the structured grid's box that the
@@ -470,25 +485,60 @@ class FemPIC:
         p.size -= remove_count
         return kind
 
-    def step(self, rnd_soa: torch.Tensor, stream=None, timers: StepTimes | None = None) -> dict:
-        """One FemPIC particle step.  Reads the move status once (the remove count that
-        sizes the compaction), as the reference does after its move."""
-        ev = [torch.cuda.Event(enable_timing=True) for _ in range(5)] if timers is not None else None
-        s = stream if stream is not None else torch.cuda.current_stream()
-        if ev: ev[0].record(s)
+    def _begin_step(self, rnd_soa: torch.Tensor, s) -> tuple:
+        """inject, charge reset, push and move of a step in one native call (oppb_step_begin);
+        returns the size before the move and its status."""
+        p = self.parts
+        count = rnd_soa.shape[1]
+        p.increase(count)
+        p.size += count
+        v = p.view()
+        a, mixed = self._step_args, self.precision == "mixed"
+        a.mesh, a.inlet, a.n_nodes = C.pointer(self.mesh.s), C.pointer(self.mesh.inlet), self.mesh.n_nodes
+        a.status, a.status_host = _ptr(p.status), self._status_pinned.data_ptr()
+        a.rnd, a.rnd_stride, a.rnd_dim, a.n_inject = _ptr(rnd_soa), rnd_soa.stride(0), rnd_soa.shape[0], count
+        a.ion_velocity, a.max_hops, a.node_charge = self.ion_velocity, self.max_hops, _ptr(self.node_charge)
+        m = a.move
+        m.precision = L.PRECISION_MIXED if mixed else L.PRECISION_F64
+        m.deposit, m.push = int(mixed or self.fused_deposit), int(self.fused_push)
+        m.qm, m.dt, m.band = self.qm, self.dt, self.band
+        if self.dh is not None:
+            m.dh = C.pointer(self.dh.g)
+        elif m.dh:
+            m.dh = None
+        a.separate_push = int(not self.fused_push)
+        ws = self._deposit_ws()
+        a.workspace, a.workspace_bytes = _ptr(ws), ws.numel()
+        L.check("oppb_step_begin", self.lib.oppb_step_begin(C.byref(a), C.byref(v), s.cuda_stream or None))
+        return p.size, self._status_host
+
+    def _begin_step_timed(self, rnd_soa: torch.Tensor, stream, s, ev) -> tuple:
+        """_begin_step with an event after each of its parts."""
+        ev[0].record(s)
         self.inject(rnd_soa, stream)
         self.zero_node_charge(stream)
-        if ev: ev[1].record(s)
+        ev[1].record(s)
         n_before = self.parts.size
         if self.fused_push:
-            if ev: ev[2].record(s)
+            ev[2].record(s)
             self.push_move(stream)  # push time is counted in move_ms
         else:
             self.push(stream)
-            if ev: ev[2].record(s)
+            ev[2].record(s)
             self.move(stream)  # unfused FP64 deposit runs after the compaction, as the reference loop order
-        if ev: ev[3].record(s)
-        st = self.parts.status_host()
+        ev[3].record(s)
+        return n_before, self.parts.status_host()
+
+    def step(self, rnd_soa: torch.Tensor, stream=None, timers: StepTimes | None = None) -> dict:
+        """One FemPIC particle step.  Reads the move status once (the remove count that
+        sizes the compaction), as the reference does after its move."""
+        s = stream if stream is not None else torch.cuda.current_stream()
+        ev = None
+        if timers is None:
+            n_before, st = self._begin_step(rnd_soa, s)
+        else:
+            ev = [torch.cuda.Event(enable_timing=True) for _ in range(5)]
+            n_before, st = self._begin_step_timed(rnd_soa, stream, s, ev)
         if st.error:
             raise L.OppbError(f"move (particle {st.error_index})", st.error)
         kind = self.finalize(st.remove_count, stream)
