@@ -60,8 +60,23 @@ __global__ void __launch_bounds__(kPushBlock) push_mixed_kernel(int32_t size, in
     }
 }
 
-// First inlet face j with k < dist[j] (the last face if none).
-__device__ __forceinline__ int face_of(const int32_t* __restrict__ dist, int32_t n_faces, int64_t k) {
+// First inlet face j with k < dist[j] (the last face if none) for particle k of count.  The faces of
+// an inlet take nearly equal shares, so the face at k's share of the faces, or one next to it, is
+// almost always the one: their bounds are read at once, where the binary search below reads one
+// after the other (8 for 200 faces, 13 for 4,608) and was most of the injection's latency.
+__device__ __forceinline__ int face_of(const int32_t* __restrict__ dist, int32_t n_faces, int64_t k, int32_t count) {
+    const int g = min(n_faces - 1, (int)(__int2float_rn((int)k) * __fdividef((float)n_faces, (float)count)));
+    int32_t d[4];  // dist[g - 2 .. g + 1]
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const int f = g - 2 + j;
+        d[j] = f < 0 ? -1 : __ldg(dist + min(f, n_faces - 1));
+    }
+#pragma unroll
+    for (int j = 1; j < 4; j++) {
+        const int f = g - 2 + j;
+        if (f >= 0 && f < n_faces && k < d[j] && k >= d[j - 1]) return f;
+    }
     int lo = 0, hi = n_faces;
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
@@ -76,7 +91,7 @@ __device__ __forceinline__ int face_of(const int32_t* __restrict__ dist, int32_t
 __global__ void __launch_bounds__(kPushBlock) assign_faces_kernel(int32_t start, int32_t count, int32_t n_faces,
                                                                   const int32_t* __restrict__ dist, int32_t* p2c) {
     const int64_t k = (int64_t)blockIdx.x * kPushBlock + threadIdx.x;
-    if (k < count) p2c[(int64_t)start + k] = face_of(dist, n_faces, k);
+    if (k < count) p2c[(int64_t)start + k] = face_of(dist, n_faces, k, count);
 }
 
 template <typename T>
@@ -110,7 +125,7 @@ __global__ void __launch_bounds__(kPushBlock) inject_kernel(oppb_set_count* cnt,
     }
     if (k >= count) return;
     // Without a distribution the face index is already in p2c (opp_inc_part_count_with_distribution).
-    const int face = dist ? face_of(dist, n_faces, k) : p2c[(int64_t)start + k];
+    const int face = dist ? face_of(dist, n_faces, k, count) : p2c[(int64_t)start + k];
     if ((uint32_t)face >= (uint32_t)n_faces) {
         p2c[(int64_t)start + k] = kRemoved;
         return;
