@@ -40,9 +40,9 @@ extern "C" {
 /* ------------------------------------------------------------------ types */
 
 /* Device-resident tetrahedral mesh in the packed layout the kernels read: one cell
- * visit of the FP64 move is four 256-bit loads of `det` and one of `nav`; of the mixed
- * move two of `geo32` (64 B), plus one 16-B read of the nav32 neighbours when the
- * particle hops on.  Filled by oppb_tet_mesh_pack(); buffers are
+ * visit of the FP64 move is four 256-bit loads of `det` and the 8-B coefficient of `nav`, plus
+ * one 4-B neighbour of it when the particle hops on; of the mixed move two of `geo32` (64 B), plus
+ * one 4-B neighbour of nav32.  det is read fastest when it starts on a 128-byte line.  Filled by oppb_tet_mesh_pack(); buffers are
  * owned by the caller and 32-byte aligned (oppb_tet_mesh_bytes gives the sizes).
  *   det   [n_cells][16] f64 : {alpha,beta,gamma,delta} of vertex 0..3
  *                             (minifempic_funcs.h:316-382 ordering), 128-B record
@@ -153,9 +153,9 @@ typedef struct oppb_tuning {
                                deposit: 128, 256 (0 reads as 256) or 512, with 2048 / move_block CTAs
                                resident per SM (32 registers a thread); the other deposits, the lane-pair
                                and the staged kernels use 256.  The same results */
-    int32_t cabana_occupancy; /* CabanaPIC move + deposit: resident CTAs per SM it is compiled for:
-                                 0 = the compiler's register count, 4 (default; 64 registers a
-                                 thread) or 5 (48 registers, small spills).  The same results */
+    int32_t cabana_occupancy; /* CabanaPIC move + deposit: resident warps per SM it is compiled for, in
+                                 units of eight: 0 = the compiler's register count, 4 (default; 64
+                                 registers a thread) or 5 (48 registers, spills).  The same results */
     int32_t move_walk32;      /* FP64 move + deposit: 1 = walk on the mixed path's FP32 records (each
                                  inside test and argmin decided in FP32 or, near a threshold, by the
                                  FP64 expression, so equal to the FP64 decision) and evaluate the FP64

@@ -103,8 +103,8 @@ int oppb_advec_step(const oppb_advec_batch* batch, oppb_move_status* status, int
 /* The two loops separately, as the generated main calls them:
  * opp_par_loop_all__update_pos_kernel (apps_codegen/app_neso_advection_mdir_cg/cuda/update_pos_kernel_loop.hpp)
  * and opp_particle_move__move_kernel (.../cuda/move_kernel_loop.hpp).  The update reads the
- * batch's pos and vel only (mdir, p2c and cells may be NULL); the move reads pos, mdir, p2c and
- * cells (vel may be NULL). */
+ * batch's pos and vel only (mdir, p2c and cells may be NULL); the move reads pos, p2c and
+ * cells and writes mdir and p2c (vel may be NULL). */
 int oppb_advec_update_pos(const oppb_advec_batch* batch, void* stream);
 int oppb_advec_move(const oppb_advec_batch* batch, oppb_move_status* status, int32_t max_hops,
                     void* stream);

@@ -100,7 +100,7 @@ int oppb_node_charge_density(double* n_charge_den, const double* n_vol, double s
 /* FESolver::compute_phi: tempNEQ1/2/3 from D and ion_den (init_f1_and_J), F1 += the cell
  * integrals of tempNEQ1 (build_f1_vector; F1 is never reset, as in the reference), the
  * diagonal of J = K - diag(integrals of tempNEQ3) (build_j_matrix), B = K D - F0 - F1, CG on
- * J Y = B (Jacobi preconditioner, one cooperative launch), D -= Y, then node_potential =
+ * J Y = B (Jacobi preconditioner, one persistent launch), D -= Y, then node_potential =
  * n_bnd_pot + D on unknowns (compute_node_potential).  ion_den, node_potential: device
  * [n_nodes].  status: device, written at the end. */
 int oppb_field_solve(const oppb_field_device* f, const oppb_field_consts* c, const double* ion_den,

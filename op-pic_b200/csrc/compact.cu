@@ -230,9 +230,10 @@ __global__ void __launch_bounds__(256) removal_bits_kernel(const int32_t* __rest
 }
 
 // Blocks up to which the emit kernel sums the blocks' counts itself instead of a scan launch (4.2 us
-// and a gap): 16 loads a thread at the limit, 67M particles.  A captured ten-step cycle of 460k
+// and a gap): 4 loads a thread at the limit, 16.8M particles (at 57M particles, 3,517 blocks, the
+// emit kernel takes 12 us longer so).  A captured ten-step cycle of 460k
 // particles takes 714 us instead of 796, a step-by-step one 525 instead of 540 (four steps).
-constexpr int kHfDirectBlocks = 4096;
+constexpr int kHfDirectBlocks = 1024;
 
 // The hole fill's launches.  block_holes: n_blocks + 1 ints.
 int launch_hole_fill(const uint32_t* remove_bits, const CountArg& sz, const CountArg& rc, int64_t n_words, int n_blocks,
@@ -305,7 +306,6 @@ extern "C" int oppb_hole_fill(int32_t size, int32_t remove_count, const uint32_t
     char* ws = static_cast<char*>(workspace);
     int* block_base = reinterpret_cast<int*>(ws);
     ws += align256(sizeof(int) * (size_t)(n_blocks + 1));
-    int* scan_tmp = reinterpret_cast<int*>(ws);
     ws += align256(sizeof(int) * scan_scratch_ints(n_blocks));
     int32_t* hole_list = reinterpret_cast<int32_t*>(ws);
     ws += align256(sizeof(int32_t) * (size_t)remove_count);

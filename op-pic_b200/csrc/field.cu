@@ -5,7 +5,8 @@
 // is compiled with -fmad=false), so their results equal the reference's bit for bit for the
 // same inputs.
 //
-// compute_phi is one cooperative launch: the grid runs init_f1_and_J, build_f1_vector and
+// compute_phi of a system kept by diagonals takes the kernels of "CG on K by diagonals" below.  Any
+// other system is one cooperative launch, field_newton_kernel: the grid runs init_f1_and_J, build_f1_vector and
 // build_j_matrix (cell integrals added with FP64 atomics, as the reference's device
 // kernels do), B = K D - F0 - F1, then Jacobi-preconditioned CG on J Y = B, D -= Y and the
 // node potentials, separated by grid-wide barriers.  The iteration count is bounded by

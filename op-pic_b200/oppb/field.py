@@ -4,7 +4,7 @@ FieldDevice holds FESolver's system on the GPU (built once on the host by
 oppb_field_setup: equation map, detJ, shape derivatives, stiffness matrix K, F0) with the
 Newton state D and the accumulated F1, and runs per step:
   node_charge_density   compute_node_charge_density_kernel (n_charge_den *= spwt / n_vol)
-  solve                 FESolver::compute_phi, one cooperative launch, no host sync
+  solve                 FESolver::compute_phi, no host sync
   electric_field        compute_electric_field_kernel into any [cell][stride] field array
 The three calls capture into one CUDA graph (capture()).
 """
