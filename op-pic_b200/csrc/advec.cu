@@ -214,8 +214,8 @@ __global__ void __launch_bounds__(kAdvBlock, kItems == 1 ? 5 : kItems == 2 ? 4 :
                 x[k] = ld_stream(b.pos + i);
                 y[k] = ld_stream(b.pos + sd + i);
                 if (kMode != kMoveOnly) {
-                    vx[k] = __ldcs(b.vel + i);
-                    vy[k] = __ldcs(b.vel + sd + i);
+                    vx[k] = __ldg(b.vel + i);  // read again next step: a small batch keeps it in L2
+                    vy[k] = __ldg(b.vel + sd + i);
                 }
                 if (kMode != kUpdateOnly) cell[k] = ld_stream(b.p2c + i);
             }
