@@ -449,6 +449,9 @@ __global__ void __launch_bounds__(kCgMaxThreads, 1) field_cg_kernel(const __grid
     double* km = dyn + width;  // [smem_diag][rows]
     double* zg = a.q;          // z of all rows, the only vector blocks exchange
     unsigned turn = 1;
+    // A block's shared memory may be written by the others only once it runs, which being scheduled
+    // together does not say: all have started before the first reduction stores into all.
+    if (kCluster) cg::this_cluster().sync();
     if (threadIdx.x == 0) sh.failed = 0;
     for (int32_t i = threadIdx.x; i < width; i += blockDim.x) pw[i] = 0.0;
     const int32_t stream_diag = a.n_diag - c.smem_diag;
