@@ -100,11 +100,25 @@ int oppb_node_charge_density(double* n_charge_den, const double* n_vol, double s
 /* FESolver::compute_phi: tempNEQ1/2/3 from D and ion_den (init_f1_and_J), F1 += the cell
  * integrals of tempNEQ1 (build_f1_vector; F1 is never reset, as in the reference), the
  * diagonal of J = K - diag(integrals of tempNEQ3) (build_j_matrix), B = K D - F0 - F1, CG on
- * J Y = B (Jacobi preconditioner, one persistent launch), D -= Y, then node_potential =
+ * J Y = B (Jacobi preconditioner), D -= Y, then node_potential =
  * n_bnd_pot + D on unknowns (compute_node_potential).  ion_den, node_potential: device
  * [n_nodes].  status: device, written at the end. */
 int oppb_field_solve(const oppb_field_device* f, const oppb_field_consts* c, const double* ion_den,
                      double* node_potential, oppb_field_status* status, void* stream);
+
+/* How a solve is launched (oppb_field_solve: OPPB_FIELD_MAX_POLLS, 0).  max_polls bounds each wait among
+ * the CG's blocks, in polls of about a microsecond; only the solve of a system by diagonals too
+ * large for one cluster polls.  If a wait runs out, the step is not taken: D keeps its values,
+ * node_potential is that of D, and the status says not converged. */
+#define OPPB_FIELD_MAX_POLLS (1 << 20)
+typedef struct oppb_field_options {
+    int32_t max_polls;
+    int32_t reserved;
+} oppb_field_options;
+
+int oppb_field_solve_ex(const oppb_field_device* f, const oppb_field_consts* c, const double* ion_den,
+                        double* node_potential, oppb_field_status* status, const oppb_field_options* options,
+                        void* stream);
 
 /* compute_electric_field_kernel over the cells after opp_reset_dat(c_ef):
  * c_ef[d] = 0 - (((sd0 phi0 + sd1 phi1) + sd2 phi2) + sd3 phi3) per dimension.  c_sd

@@ -126,11 +126,11 @@ __device__ __forceinline__ void add_cell_integrals(const FieldArgs& a, int64_t t
     }
 }
 
-// compute_node_potential.
-__device__ __forceinline__ void node_potentials(const FieldArgs& a, int64_t tid, int64_t nth) {
+// compute_node_potential from D's values d.
+__device__ __forceinline__ void node_potentials(const FieldArgs& a, const double* d, int64_t tid, int64_t nth) {
     for (int64_t n = tid; n < a.n_nodes; n += nth) {
         const int32_t e = a.node_to_eq[n];
-        a.potential[n] = a.n_bnd_pot[n] + ((e >= 0) ? a.d[e] : 0);
+        a.potential[n] = a.n_bnd_pot[n] + ((e >= 0) ? d[e] : 0);
     }
 }
 
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(kFieldBlock) field_newton_kernel(FieldArgs a) 
     // D -= Y (VecAXPY(D, -1, Y)), then compute_node_potential.
     for (int64_t u = tid; u < a.neq; u += nth) a.d[u] = a.d[u] - a.x[u];
     grid.sync();
-    node_potentials(a, tid, nth);
+    node_potentials(a, a.d, tid, nth);
     if (tid == 0) {
         a.status->iterations = it;
         a.status->converged = sqrt(rr) <= stop;
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(kFieldBlock) field_newton_kernel(FieldArgs a) 
 // ------------------------------------------------------------- CG on K by diagonals
 //
 // The Newton step of a system stored by diagonals: two set-up kernels over the whole chip, one
-// persistent CG kernel, one kernel for the node potentials.
+// persistent CG kernel, one kernel that takes the step and writes the node potentials.
 //
 // What bounds the CG is neither DRAM nor arithmetic but what an iteration does one after the
 // other: grid barriers, passes over vectors in memory and the loads of K.  So each block owns a
@@ -307,7 +307,6 @@ constexpr int kCgMaxCluster = 16;
 constexpr int kCgMaxWarps = kCgMaxThreads / 32;
 constexpr int kCgMaxBlocks = 160;  // of the grid form
 
-constexpr int kCgMaxPolls = 1 << 20;  // about a second
 
 // One block's sums in global memory: each value and the number of the reduction it belongs to are
 // one 16-byte word, so that a block that reads the number has the value too.  A slot fills a
@@ -346,7 +345,10 @@ struct CgArgs {
     int32_t rows;      // rows a block owns
     int32_t lo, hi;    // the window reaches lo rows before and hi rows after them
     int32_t smem_diag; // the last smem_diag diagonals are kept in shared memory
+    int32_t max_polls; // bound of a wait of the grid form
     CgSlot* slots;     // [2][gridDim.x], grid form; zeroed before the launch
+    int* gave_up;      // 1 once a block's wait has run out; zeroed before the launch
+    double* next_d;    // [neq] D - Y
 };
 
 // Sums over the lanes that hold one value: all 32 for kValues = 1, else lanes 0..15 hold the first
@@ -367,9 +369,10 @@ __device__ __forceinline__ double lane_sum(double v) {
 // then one cluster barrier.  Grid form: the block's sums go to its slot together with the turn, and
 // warp 0 polls the slots of all blocks, so that the reduction and the barrier are one round trip
 // through L2 (a cooperative-groups grid barrier with the partial sums beside it took 7 us).  The
-// blocks are all resident (cooperative launch); a wait that runs out sets sh.failed.
+// blocks are all resident (cooperative launch); a wait that runs out sets sh.failed, on which the block
+// ends, and *gave_up, on which field_finish_kernel drops the step of all blocks.
 template <int kValues, bool kBarrier, bool kCluster>
-__device__ __forceinline__ double2 cg_all_sum(double2 in, CgShared& sh, CgSlot* slots, unsigned turn) {
+__device__ __forceinline__ double2 cg_all_sum(double2 in, CgShared& sh, const CgArgs& c, unsigned turn) {
     constexpr int kLanes = 32 / kValues;  // lanes a value
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
     const int sub = lane % kLanes, value = lane / kLanes;
@@ -404,15 +407,15 @@ __device__ __forceinline__ double2 cg_all_sum(double2 in, CgShared& sh, CgSlot* 
         v = 0.0;
         for (int w = sub; w < n_warps; w += kLanes) v += sh.warp[value][w];
         v = lane_sum<kValues>(v);
-        CgSlot* at = slots + (turn & 1) * n_blocks;
+        CgSlot* at = c.slots + (turn & 1) * n_blocks;
         if (sub == 0) {
             if (kBarrier) __threadfence();
             post_word(&at[blockIdx.x].value[value], v, turn);
         }
         constexpr int kSlots = (kCgMaxBlocks + kLanes - 1) / kLanes;
-        double x[kSlots];
+        double x[kSlots] = {};
         bool all = false;
-        for (int poll = 0; !all && poll < kCgMaxPolls; poll++) {
+        for (int poll = 0; !all && poll < c.max_polls; poll++) {
             bool here = true;
 #pragma unroll
             for (int k = 0; k < kSlots; k++) {
@@ -431,7 +434,7 @@ __device__ __forceinline__ double2 cg_all_sum(double2 in, CgShared& sh, CgSlot* 
         for (int k = 0; k < kSlots; k++) v += x[k];
         v = lane_sum<kValues>(v);
         if (sub == 0) sh.sum[value] = v;
-        if (lane == 0 && !all) sh.failed = 1;
+        if (lane == 0 && !all) sh.failed = *c.gave_up = 1;
     }
     __syncthreads();
     return make_double2(sh.sum[0], kValues == 2 ? sh.sum[1] : 0.0);
@@ -482,13 +485,14 @@ __global__ void __launch_bounds__(kCgMaxThreads, 1) field_cg_kernel(const __grid
         v.x += r[k] * z[k];
         v.y += r[k] * r[k];
     }
-    v = cg_all_sum<2, true, kCluster>(v, sh, c.slots, turn++);
+    v = cg_all_sum<2, true, kCluster>(v, sh, c, turn++);
     double rz = v.x, rr = v.y;
     const double b_norm = sqrt(rr);
     const double stop = fmax(a.rtol * b_norm, a.atol);
     double beta = 0.0;
     int it = 0;
-    while (it < a.max_iter && sqrt(rr) > stop) {
+    bool failed = !kCluster && sh.failed;
+    while (!failed && it < a.max_iter && sqrt(rr) > stop) {
         // p = z + beta p over the window: the block's own rows from registers, the rest with kStage
         // loads of z in flight a thread.
         const int32_t halo = c.lo + c.hi;
@@ -555,8 +559,9 @@ __global__ void __launch_bounds__(kCgMaxThreads, 1) field_cg_kernel(const __grid
             const int32_t i = threadIdx.x + k * blockDim.x;
             if (i < n_own) v.x += pw[i + c.lo] * s[k];
         }
-        v = cg_all_sum<1, false, kCluster>(v, sh, c.slots, turn++);
-        if (!kCluster && sh.failed) break;
+        v = cg_all_sum<1, false, kCluster>(v, sh, c, turn++);
+        failed = !kCluster && sh.failed;
+        if (failed) break;
         const double alpha = rz / v.x;
         v = make_double2(0.0, 0.0);
 #pragma unroll
@@ -570,32 +575,33 @@ __global__ void __launch_bounds__(kCgMaxThreads, 1) field_cg_kernel(const __grid
             v.x += r[k] * z[k];
             v.y += r[k] * r[k];
         }
-        v = cg_all_sum<2, true, kCluster>(v, sh, c.slots, turn++);
-        if (!kCluster && sh.failed) break;
+        v = cg_all_sum<2, true, kCluster>(v, sh, c, turn++);
+        failed = !kCluster && sh.failed;
+        if (failed) break;
         beta = v.x / rz;
         rz = v.x;
         rr = v.y;
         it++;
     }
-    const bool failed = !kCluster && sh.failed;
-    // D -= Y (VecAXPY(D, -1, Y)).
+    // D - Y (VecAXPY(D, -1, Y)), which field_finish_kernel makes D.
 #pragma unroll
     for (int k = 0; k < kRows; k++) {
         const int32_t i = threadIdx.x + k * blockDim.x;
-        if (i < n_own && !failed) a.d[r0 + i] = a.d[r0 + i] - x[k];
+        if (i < n_own) c.next_d[r0 + i] = a.d[r0 + i] - x[k];
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         a.status->iterations = it;
-        a.status->converged = !failed && sqrt(rr) <= stop;
+        a.status->converged = sqrt(rr) <= stop;
         a.status->resid = b_norm > 0.0 ? sqrt(rr) / b_norm : 0.0;
         a.status->b_norm = b_norm;
     }
 }
 
 __global__ void __launch_bounds__(kFieldBlock) field_init_kernel(const __grid_constant__ FieldArgs a,
-                                                                  CgSlot* slots, int n_slots) {
+                                                                  CgSlot* slots, int n_slots, int* gave_up) {
     if ((int)(blockIdx.x * kFieldBlock + threadIdx.x) < n_slots)
         slots[blockIdx.x * kFieldBlock + threadIdx.x] = CgSlot{};
+    if (blockIdx.x == 0 && threadIdx.x == 0) *gave_up = 0;
     init_terms(a, (int64_t)blockIdx.x * kFieldBlock + threadIdx.x, (int64_t)gridDim.x * kFieldBlock);
 }
 
@@ -603,8 +609,17 @@ __global__ void __launch_bounds__(kFieldBlock) field_cells_kernel(const __grid_c
     add_cell_integrals(a, (int64_t)blockIdx.x * kFieldBlock + threadIdx.x, (int64_t)gridDim.x * kFieldBlock);
 }
 
-__global__ void __launch_bounds__(kFieldBlock) field_potential_kernel(const __grid_constant__ FieldArgs a) {
-    node_potentials(a, (int64_t)blockIdx.x * kFieldBlock + threadIdx.x, (int64_t)gridDim.x * kFieldBlock);
+// D and the node potentials of the step, unless a block of field_cg_kernel gave up: then D stays as it
+// was, whichever blocks ended their CG, and the status says not converged.
+__global__ void __launch_bounds__(kFieldBlock) field_finish_kernel(const __grid_constant__ FieldArgs a, const int* gave_up,
+                                                                    const double* next_d) {
+    const int64_t tid = (int64_t)blockIdx.x * kFieldBlock + threadIdx.x, nth = (int64_t)gridDim.x * kFieldBlock;
+    const bool failed = *gave_up != 0;
+    node_potentials(a, failed ? a.d : next_d, tid, nth);
+    if (!failed)
+        for (int64_t u = tid; u < a.neq; u += nth) a.d[u] = next_d[u];
+    else if (tid == 0)
+        a.status->converged = 0;
 }
 
 __global__ void __launch_bounds__(256) node_charge_density_kernel(double* den, const double* vol, double spwt,
@@ -761,12 +776,14 @@ int make_cg_plan(const FieldArgs& a, CgPlan* plan, int32_t* lo, int32_t* hi) {
     return OPPB_OK;
 }
 
-int solve_by_diagonals(const FieldArgs& a, const CgPlan& p, int32_t lo, int32_t hi, cudaStream_t s) {
+int solve_by_diagonals(const FieldArgs& a, const CgPlan& p, int32_t lo, int32_t hi, int32_t max_polls, cudaStream_t s) {
     const int most = 148 * 8;
     const int eq_grid = ceil_div(a.n_nodes, kFieldBlock), cell_grid = ceil_div(a.n_cells, kFieldBlock);
     CgArgs c{};
     c.f = a;
-    c.rows = p.rows, c.lo = lo, c.hi = hi, c.smem_diag = p.smem_diag;
+    c.rows = p.rows, c.lo = lo, c.hi = hi, c.smem_diag = p.smem_diag, c.max_polls = max_polls;
+    c.next_d = a.diag;  // of the work space too: this path keeps the diagonal in registers
+    c.gave_up = reinterpret_cast<int*>(a.partial_a);
     // The slots lie in the vectors x, r and p of the work space, which this path keeps on chip:
     // 32 doubles a block of at least kCgMinRows rows, and the alignment.
     static_assert(3 * kCgMinRows >= 32 + 16, "the slots fit");
@@ -774,11 +791,11 @@ int solve_by_diagonals(const FieldArgs& a, const CgPlan& p, int32_t lo, int32_t 
     const int n_slots = p.cluster ? 0 : 2 * p.blocks;
     const int slot_grid = ceil_div(n_slots, kFieldBlock);
     const int init_grid = eq_grid < most ? (eq_grid > slot_grid ? eq_grid : slot_grid) : most;
-    field_init_kernel<<<init_grid, kFieldBlock, 0, s>>>(a, c.slots, n_slots);
+    field_init_kernel<<<init_grid, kFieldBlock, 0, s>>>(a, c.slots, n_slots, c.gave_up);
     field_cells_kernel<<<cell_grid, kFieldBlock, 0, s>>>(a);
     const int rc = p.cluster ? launch_cg_rows<true>(p, c, s) : launch_cg_rows<false>(p, c, s);
     if (rc) return rc;
-    field_potential_kernel<<<eq_grid < most ? eq_grid : most, kFieldBlock, 0, s>>>(a);
+    field_finish_kernel<<<eq_grid < most ? eq_grid : most, kFieldBlock, 0, s>>>(a, c.gave_up, c.next_d);
     count_launches(4);
     return launch_status();
 }
@@ -860,10 +877,11 @@ extern "C" int oppb_reduce_max(const double* x, int64_t n, int32_t absolute, dou
     return oppb::launch_status();
 }
 
-extern "C" int oppb_field_solve(const oppb_field_device* f, const oppb_field_consts* c, const double* ion_den,
-                                double* node_potential, oppb_field_status* status, void* stream) {
+extern "C" int oppb_field_solve_ex(const oppb_field_device* f, const oppb_field_consts* c, const double* ion_den,
+                                   double* node_potential, oppb_field_status* status, const oppb_field_options* options,
+                                   void* stream) {
     using namespace oppb;
-    if (!f || !c || !ion_den || !node_potential || !status) return OPPB_ERR_ARG;
+    if (!f || !c || !ion_den || !node_potential || !status || !options || options->max_polls < 0) return OPPB_ERR_ARG;
     if (f->n_nodes <= 0 || f->n_cells <= 0 || f->neq < 0 || !f->node_to_eq || !f->c2n || !f->det_j ||
         !f->n_bnd_pot || !f->k_rowptr || !f->d || !f->f1 || !f->work || !f->f0 || (f->neq > 0 && (!f->k_col ||
         !f->k_val)))
@@ -891,7 +909,7 @@ extern "C" int oppb_field_solve(const oppb_field_device* f, const oppb_field_con
     int32_t lo = 0, hi = 0;
     int rc = make_cg_plan(a, &plan, &lo, &hi);
     if (rc) return rc;
-    if (plan.rows) return solve_by_diagonals(a, plan, lo, hi, as_stream(stream));
+    if (plan.rows) return solve_by_diagonals(a, plan, lo, hi, options->max_polls, as_stream(stream));
     int blocks = 0;
     if ((rc = coop_grid(&blocks))) return rc;
     void* args[] = {&a};
@@ -900,4 +918,10 @@ extern "C" int oppb_field_solve(const oppb_field_device* f, const oppb_field_con
         return OPPB_ERR_LAUNCH;
     count_launches(1);
     return launch_status();
+}
+
+extern "C" int oppb_field_solve(const oppb_field_device* f, const oppb_field_consts* c, const double* ion_den,
+                                double* node_potential, oppb_field_status* status, void* stream) {
+    const oppb_field_options options{OPPB_FIELD_MAX_POLLS, 0};
+    return oppb_field_solve_ex(f, c, ion_den, node_potential, status, &options, stream);
 }

@@ -146,6 +146,10 @@ class FieldStatus(C.Structure):
     _fields_ = [("iterations", c_i32), ("converged", c_i32), ("resid", C.c_double), ("b_norm", C.c_double)]
 
 
+class FieldOptions(C.Structure):
+    _fields_ = [("max_polls", c_i32), ("reserved", c_i32)]
+
+
 class FemPICMesh(C.Structure):
     _fields_ = [("n_nodes", c_i32), ("n_cells", c_i32), ("n_ifaces", c_i32),
                 ("n_pos", c_dp), ("n_vol", c_dp), ("n_type", c_ip), ("n_bnd_pot", c_dp),
@@ -229,6 +233,7 @@ _SIGS = {
     "oppb_field_work_doubles": (C.c_size_t, [c_i32]),
     "oppb_node_charge_density": (C.c_int, [c_vp, c_vp, C.c_double, c_i32, c_vp]),
     "oppb_field_solve": (C.c_int, [P(FieldDevice), P(FieldConsts), c_vp, c_vp, c_vp, c_vp]),
+    "oppb_field_solve_ex": (C.c_int, [P(FieldDevice), P(FieldConsts), c_vp, c_vp, c_vp, P(FieldOptions), c_vp]),
     "oppb_electric_field": (C.c_int, [c_vp, c_vp, c_vp, c_vp, c_i32, c_i32, c_vp]),
     "oppb_fempic_box_mesh": (C.c_int, [c_i32, c_i32, c_i32, C.c_double, C.c_double, C.c_double, P(FemPICMesh)]),
     "oppb_fempic_solve_field": (C.c_int, [P(FemPICMesh), C.c_double, C.c_double, C.c_double, c_i32, c_dp,

@@ -48,15 +48,19 @@ class Banded:
                 s.dia_off[j] = int(o)
         return s
 
-    def launch(self, diagonals: bool = True, max_iter: int = 4000, stream=None) -> int:
-        """One solve from D = 0 and F1 = 0; returns the status code of the call."""
+    def launch(self, diagonals: bool = True, max_iter: int = 4000, stream=None, d0: float = 0.0,
+               max_polls: int | None = None) -> int:
+        """One solve from D = d0 and F1 = 0; returns the status code of the call."""
         with torch.cuda.stream(stream):
-            self.d.zero_()
+            self.d.fill_(d0)
             self.f1.zero_()
         c = L.FieldConsts(1.0, 0.0, 100.0, 1.0, 1.0, 1e-10, 1e-10, max_iter, 0)
-        return self.lib.oppb_field_solve(C.byref(self.struct(diagonals)), C.byref(c), self.ion.data_ptr(),
-                                         self.pot.data_ptr(), self.status.data_ptr(),
-                                         stream.cuda_stream if stream is not None else None)
+        args = [C.byref(self.struct(diagonals)), C.byref(c), self.ion.data_ptr(), self.pot.data_ptr(),
+                self.status.data_ptr()]
+        s = stream.cuda_stream if stream is not None else None
+        if max_polls is None:
+            return self.lib.oppb_field_solve(*args, s)
+        return self.lib.oppb_field_solve_ex(*args, C.byref(L.FieldOptions(max_polls, 0)), s)
 
     def solve(self, diagonals: bool = True, **kw) -> tuple[torch.Tensor, L.FieldStatus]:
         L.check("oppb_field_solve", self.launch(diagonals, **kw))
