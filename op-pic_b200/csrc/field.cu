@@ -686,6 +686,7 @@ struct CgPlan {
     int rows_thread = 0;
     int smem_diag = 0;
     size_t smem = 0;
+    int smem_max = 0;   // what the device gives a block
     bool cluster = false;
 };
 
@@ -697,6 +698,7 @@ constexpr int kClusterNeq = 18432;
 CgPlan cg_plan(int32_t neq, int32_t n_diag, int32_t lo, int32_t hi, int sms, int smem_max, bool cluster) {
     CgPlan p;
     p.cluster = cluster;
+    p.smem_max = smem_max;
     const int most = cluster ? kCgMaxCluster : sms < kCgMaxBlocks ? sms : kCgMaxBlocks;
     p.rows = ceil_div(neq, most);
     if (p.rows < kCgMinRows) p.rows = kCgMinRows;
@@ -714,7 +716,9 @@ CgPlan cg_plan(int32_t neq, int32_t n_diag, int32_t lo, int32_t hi, int sms, int
 template <int kRows, bool kCluster>
 int launch_cg(const CgPlan& p, CgArgs& c, cudaStream_t s) {
     auto kernel = field_cg_kernel<kRows, kCluster>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess)
+    // The attribute is the kernel's, for all threads and graphs: always the device's most, so that the
+    // solve of a smaller system cannot take it back between another's call here and its launch.
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem_max) != cudaSuccess)
         return OPPB_ERR_LAUNCH;
     if (kCluster && p.blocks > 8 &&
         cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
