@@ -694,6 +694,7 @@ struct CgPlan {
 // iteration, cluster / grid: 4.3 / 6.1 at 4,719 unknowns, 6.1 / 6.4 at 18,207, 9.0 / 6.3 at 34,839
 // (all in field_newton_kernel: 12.9, 13.7, 13.4).
 constexpr int kClusterNeq = 18432;
+static_assert(kClusterNeq <= kCgMaxCluster * kCgMaxThreads * 2, "a cluster's threads have one or two rows");
 
 CgPlan cg_plan(int32_t neq, int32_t n_diag, int32_t lo, int32_t hi, int sms, int smem_max, bool cluster) {
     CgPlan p;
@@ -713,8 +714,13 @@ CgPlan cg_plan(int32_t neq, int32_t n_diag, int32_t lo, int32_t hi, int sms, int
     return p;
 }
 
+// field_cg_kernel's launch by a plan: its attributes set and its configuration filled in.
+struct CgLaunch {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+};
 template <int kRows, bool kCluster>
-int launch_cg(const CgPlan& p, CgArgs& c, cudaStream_t s) {
+int prepare_cg(const CgPlan& p, CgLaunch& l, cudaStream_t s) {
     auto kernel = field_cg_kernel<kRows, kCluster>;
     // The attribute is the kernel's, for all threads and graphs: always the device's most, so that the
     // solve of a smaller system cannot take it back between another's call here and its launch.
@@ -723,23 +729,42 @@ int launch_cg(const CgPlan& p, CgArgs& c, cudaStream_t s) {
     if (kCluster && p.blocks > 8 &&
         cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
         return OPPB_ERR_LAUNCH;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(p.blocks);
-    cfg.blockDim = dim3(p.threads);
-    cfg.dynamicSmemBytes = p.smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr{};
+    l.cfg.gridDim = dim3(p.blocks);
+    l.cfg.blockDim = dim3(p.threads);
+    l.cfg.dynamicSmemBytes = p.smem;
+    l.cfg.stream = s;
     if (kCluster) {
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = (unsigned)p.blocks;
-        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        l.attr.id = cudaLaunchAttributeClusterDimension;
+        l.attr.val.clusterDim.x = (unsigned)p.blocks;
+        l.attr.val.clusterDim.y = l.attr.val.clusterDim.z = 1;
     } else {
-        attr.id = cudaLaunchAttributeCooperative;
-        attr.val.cooperative = 1;
+        l.attr.id = cudaLaunchAttributeCooperative;
+        l.attr.val.cooperative = 1;
     }
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, c) == cudaSuccess ? OPPB_OK : OPPB_ERR_LAUNCH;
+    l.cfg.attrs = &l.attr;
+    l.cfg.numAttrs = 1;
+    return OPPB_OK;
+}
+
+template <int kRows, bool kCluster>
+int launch_cg(const CgPlan& p, CgArgs& c, cudaStream_t s) {
+    CgLaunch l;
+    const int rc = prepare_cg<kRows, kCluster>(p, l, s);
+    if (rc) return rc;
+    return cudaLaunchKernelEx(&l.cfg, field_cg_kernel<kRows, kCluster>, c) == cudaSuccess ? OPPB_OK : OPPB_ERR_LAUNCH;
+}
+
+// Whether the device can place the plan's cluster: 16 blocks with most of an SM's shared memory each need
+// as many SMs of one GPC, which a partition of the GPU may not have.
+template <int kRows>
+bool cluster_fits(const CgPlan& p) {
+    CgLaunch l;
+    int clusters = 0;
+    if (prepare_cg<kRows, true>(p, l, nullptr) == OPPB_OK &&
+        cudaOccupancyMaxActiveClusters(&clusters, field_cg_kernel<kRows, true>, &l.cfg) == cudaSuccess && clusters > 0)
+        return true;
+    cudaGetLastError();  // the answer is no, not an error of this call
+    return false;
 }
 
 template <bool kCluster>
@@ -756,8 +781,10 @@ int launch_cg_rows(const CgPlan& p, CgArgs& c, cudaStream_t s) {
     }
 }
 
-// The plan for this system on the current device; rows = 0 when it takes field_newton_kernel.
-int make_cg_plan(const FieldArgs& a, CgPlan* plan, int32_t* lo, int32_t* hi) {
+// The plan for this system on the current device; rows = 0 when it takes field_newton_kernel.  A system
+// whose cluster cannot be placed takes the grid form, from kCgMinRows unknowns on (below, the slots
+// would not fit in its work space).
+int make_cg_plan(const FieldArgs& a, bool no_cluster, CgPlan* plan, int32_t* lo, int32_t* hi) {
     *plan = CgPlan{};
     if (a.n_diag <= 0 || a.neq <= 0) return OPPB_OK;
     int64_t first = 0, last = 0;
@@ -775,8 +802,11 @@ int make_cg_plan(const FieldArgs& a, CgPlan* plan, int32_t* lo, int32_t* hi) {
         cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
         return OPPB_ERR_LAUNCH;
     smem -= (int)sizeof(CgShared) + 64;  // the kernel's static part
-    if (a.neq <= kClusterNeq) *plan = cg_plan(a.neq, a.n_diag, *lo, *hi, sms, smem, true);
-    if (!plan->rows && coop) *plan = cg_plan(a.neq, a.n_diag, *lo, *hi, sms, smem, false);
+    if (a.neq <= kClusterNeq && !no_cluster) {
+        *plan = cg_plan(a.neq, a.n_diag, *lo, *hi, sms, smem, true);
+        if (plan->rows && !(plan->rows_thread == 1 ? cluster_fits<1>(*plan) : cluster_fits<2>(*plan))) *plan = CgPlan{};
+    }
+    if (!plan->rows && coop && a.neq >= kCgMinRows) *plan = cg_plan(a.neq, a.n_diag, *lo, *hi, sms, smem, false);
     return OPPB_OK;
 }
 
@@ -789,8 +819,8 @@ int solve_by_diagonals(const FieldArgs& a, const CgPlan& p, int32_t lo, int32_t 
     c.next_d = a.diag;  // of the work space too: this path keeps the diagonal in registers
     c.gave_up = reinterpret_cast<int*>(a.partial_a);
     // The slots lie in the vectors x, r and p of the work space, which this path keeps on chip:
-    // 32 doubles a block of at least kCgMinRows rows, and the alignment.
-    static_assert(3 * kCgMinRows >= 32 + 16, "the slots fit");
+    // 32 doubles a block of kCgMinRows rows or more, a last one with fewer, and the alignment.
+    static_assert(3 * kCgMinRows >= 2 * 32 + 16, "the slots fit");
     c.slots = reinterpret_cast<CgSlot*>((reinterpret_cast<uintptr_t>(a.x) + 127) & ~(uintptr_t)127);
     const int n_slots = p.cluster ? 0 : 2 * p.blocks;
     const int slot_grid = ceil_div(n_slots, kFieldBlock);
@@ -911,7 +941,7 @@ extern "C" int oppb_field_solve_ex(const oppb_field_device* f, const oppb_field_
     a.dia_val = f->dia_val;
     CgPlan plan;
     int32_t lo = 0, hi = 0;
-    int rc = make_cg_plan(a, &plan, &lo, &hi);
+    int rc = make_cg_plan(a, options->no_cluster != 0, &plan, &lo, &hi);
     if (rc) return rc;
     if (plan.rows) return solve_by_diagonals(a, plan, lo, hi, options->max_polls, as_stream(stream));
     int blocks = 0;

@@ -147,7 +147,7 @@ class FieldStatus(C.Structure):
 
 
 class FieldOptions(C.Structure):
-    _fields_ = [("max_polls", c_i32), ("reserved", c_i32)]
+    _fields_ = [("max_polls", c_i32), ("no_cluster", c_i32)]
 
 
 class FemPICMesh(C.Structure):

@@ -49,7 +49,7 @@ class Banded:
         return s
 
     def launch(self, diagonals: bool = True, max_iter: int = 4000, stream=None, d0: float = 0.0,
-               max_polls: int | None = None) -> int:
+               max_polls: int | None = None, no_cluster: bool = False) -> int:
         """One solve from D = d0 and F1 = 0; returns the status code of the call."""
         with torch.cuda.stream(stream):
             self.d.fill_(d0)
@@ -58,9 +58,10 @@ class Banded:
         args = [C.byref(self.struct(diagonals)), C.byref(c), self.ion.data_ptr(), self.pot.data_ptr(),
                 self.status.data_ptr()]
         s = stream.cuda_stream if stream is not None else None
-        if max_polls is None:
+        if max_polls is None and not no_cluster:
             return self.lib.oppb_field_solve(*args, s)
-        return self.lib.oppb_field_solve_ex(*args, C.byref(L.FieldOptions(max_polls, 0)), s)
+        options = L.FieldOptions(1 << 20 if max_polls is None else max_polls, int(no_cluster))
+        return self.lib.oppb_field_solve_ex(*args, C.byref(options), s)
 
     def solve(self, diagonals: bool = True, **kw) -> tuple[torch.Tensor, L.FieldStatus]:
         L.check("oppb_field_solve", self.launch(diagonals, **kw))
