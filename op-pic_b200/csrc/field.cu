@@ -767,17 +767,17 @@ bool cluster_fits(const CgPlan& p) {
     return false;
 }
 
-template <bool kCluster>
 int launch_cg_rows(const CgPlan& p, CgArgs& c, cudaStream_t s) {
+    if (p.cluster) return p.rows_thread == 1 ? launch_cg<1, true>(p, c, s) : launch_cg<2, true>(p, c, s);
     switch (p.rows_thread) {
-        case 1: return launch_cg<1, kCluster>(p, c, s);
-        case 2: return launch_cg<2, kCluster>(p, c, s);
-        case 3: return launch_cg<3, kCluster>(p, c, s);
-        case 4: return launch_cg<4, kCluster>(p, c, s);
-        case 5: return launch_cg<5, kCluster>(p, c, s);
-        case 6: return launch_cg<6, kCluster>(p, c, s);
-        case 7: return launch_cg<7, kCluster>(p, c, s);
-        default: return launch_cg<8, kCluster>(p, c, s);
+        case 1: return launch_cg<1, false>(p, c, s);
+        case 2: return launch_cg<2, false>(p, c, s);
+        case 3: return launch_cg<3, false>(p, c, s);
+        case 4: return launch_cg<4, false>(p, c, s);
+        case 5: return launch_cg<5, false>(p, c, s);
+        case 6: return launch_cg<6, false>(p, c, s);
+        case 7: return launch_cg<7, false>(p, c, s);
+        default: return launch_cg<8, false>(p, c, s);
     }
 }
 
@@ -827,7 +827,7 @@ int solve_by_diagonals(const FieldArgs& a, const CgPlan& p, int32_t lo, int32_t 
     const int init_grid = eq_grid < most ? (eq_grid > slot_grid ? eq_grid : slot_grid) : most;
     field_init_kernel<<<init_grid, kFieldBlock, 0, s>>>(a, c.slots, n_slots, c.gave_up);
     field_cells_kernel<<<cell_grid, kFieldBlock, 0, s>>>(a);
-    const int rc = p.cluster ? launch_cg_rows<true>(p, c, s) : launch_cg_rows<false>(p, c, s);
+    const int rc = launch_cg_rows(p, c, s);
     if (rc) return rc;
     field_finish_kernel<<<eq_grid < most ? eq_grid : most, kFieldBlock, 0, s>>>(a, c.gave_up, c.next_d);
     count_launches(4);
