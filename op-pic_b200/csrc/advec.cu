@@ -32,19 +32,36 @@ __device__ __forceinline__ int find_instance(const int32_t* __restrict__ prefix,
     return cursor;
 }
 
-// update_pos_kernel for one axis: x += v dt, then the periodic wrap by trunc(temp / extent), the
-// quotient correctly rounded.  inv = 1 / extent: where temp * inv lies at least 2^-20 from an
-// integer (its error is below 2^30 * 2^-51) the truncation is the divide's, and the divide, some
-// twenty instructions of a kernel that issue bounds as much as DRAM, is only made next to one.
+// The quotient of update_pos_kernel's wrap: by a divide, by a reciprocal of the extent that the block
+// keeps, or by one made for the particle.
+enum Wrap { kDivide = 0, kKeptReciprocal = 1, kOwnReciprocal = 2 };
+
+// update_pos_kernel for one axis: x += v dt, then the periodic wrap temp - extent trunc(temp / extent), the
+// quotient correctly rounded.  With a reciprocal the quotient q's error is below 2^-21, so where q lies
+// at least 2^-20 from an integer its truncation is the divide's, and the divide, some twenty
+// instructions of a kernel that issue bounds as much as DRAM, is left for the other particles (2 in
+// a million).  kKeptReciprocal: inv = 1 / extent, rounded once, q < 2^30.  kOwnReciprocal: one Newton step from
+// the FP32 reciprocal y; the step's residual e is y's relative error, so with |e| < 2^-20 that of q is
+// below 2^-39, q < 2^18.  Extents past FP32 fail the test of e.
+template <int kWrap>
 __device__ __forceinline__ double update_axis(double x, double v, double dt, double extent, double inv) {
     const double offset = v * dt;
     x += offset;
     const int n_extent_offset_int = __double2int_rz(fabs(x) + 2.0);
     const double temp_pos = x + (double)n_extent_offset_int * extent;
+    if (kWrap == kDivide) return temp_pos - extent * trunc(__ddiv_rn(temp_pos, extent));
+    double e = 0.0;
+    if (kWrap == kOwnReciprocal) {
+        const double y = (double)__fdividef(1.0f, (float)extent);
+        e = __fma_rn(-extent, y, 1.0);
+        inv = __fma_rn(y, e, y);
+    }
     const double q = temp_pos * inv;
     double k = trunc(q);
     const double f = q - k;
-    if (!(f > 0x1p-20 && f < 1.0 - 0x1p-20 && q < 0x1p30)) k = trunc(__ddiv_rn(temp_pos, extent));
+    const bool sure = f > 0x1p-20 && f < 1.0 - 0x1p-20 &&
+                      (kWrap == kOwnReciprocal ? q < 0x1p18 && fabs(e) < 0x1p-20 : q < 0x1p30);
+    if (!sure) k = trunc(__ddiv_rn(temp_pos, extent));
     return temp_pos - extent * k;
 }
 
@@ -101,16 +118,9 @@ __device__ __forceinline__ int move_particle(const double* __restrict__ cells, i
 // index instead of read from the record, which oppb_advec_check_grid found equal to them bit
 // for bit.  The walk keeps (ix, iy) and steps them with the periodic wrap; the arithmetic
 // and the decisions are move_particle's.
-// inv_nx = 1 / nx: (cell + 0.5) / nx is half a cell away from an integer, so truncating the product
-// gives cell / nx.
-__device__ __forceinline__ int move_particle_grid(int32_t nx, int32_t ny, double inv_nx, int32_t n_cells, double x, double y,
-                                                  int& mx, int& my, int32_t& cell, double cw, double ex, double ey,
-                                                  int32_t max_hops, int& err) {
-    if ((uint32_t)cell >= (uint32_t)n_cells) {
-        err = OPPB_ERR_CELL_RANGE;
-        return 0;
-    }
-    int32_t iy = __double2int_rz(((double)cell + 0.5) * inv_nx);
+// iy = cell / nx.
+__device__ __forceinline__ int move_particle_grid(int32_t nx, int32_t ny, int32_t iy, double x, double y, int& mx, int& my,
+                                                  int32_t& cell, double cw, double ex, double ey, int32_t max_hops, int& err) {
     int32_t ix = cell - iy * nx;
     double dx = x - (double)ix * cw;  // c_pos_ll = (x * cell_width, y * cell_width)
     double dy = y - (double)iy * cw;
@@ -165,14 +175,20 @@ __device__ __forceinline__ int32_t dh_seed_2d(const oppb_advec_dh& g, double x, 
 // A block takes a chunk of work items from the batch's counter (so items are processed in
 // order across the whole GPU) and walks it kItems items per pass (one particle of each per
 // thread), so every thread has kItems independent particles' loads in flight.  kOnce: the grid
-// has a block for every chunk, which then is the block's only one and needs no counter.
+// has a block for every chunk, which then is the block's only one and needs no counter.  kGrid: all
+// instances are grids (oppb_advec_step_grid).
 //
-// Bound by DRAM with issue close behind (665M particles: 8.70 ms a step, 75 % of the measured copy
-// bandwidth for the 64 B a particle; 9.74 with the direction read and the divides made).  The
+// Bound by DRAM with issue close behind (665M particles of grids: 9.0 ms a step, 73 % of the measured
+// copy bandwidth for the 64 B a particle; 9.7 with the direction read and the divides made).  The
 // move direction is not read: move_kernel's first call (OPP_DO_ONCE) overwrites it.
-template <int kMode, int kItems, bool kSeed, bool kOnce>
-__global__ void __launch_bounds__(kAdvBlock, kItems == 1 ? 5 : kItems == 2 ? 4 : 2) advec_kernel(oppb_advec_batch b, oppb_move_status* st,
-                                                          int32_t max_hops, int32_t chunk_items) {
+//
+// Two particles a thread leave the step no register of its 64, so the walk over records keeps nothing
+// between particles.  Ten steps of 9.0M particles, microseconds: records 1,514 (1,571 with reciprocals
+// kept in one kernel for both forms), with the global move 1,769 (1,930); grids 1,230 (1,251), with
+// the global move 1,429 (1,546; 1,539 with the extents' reciprocals kept instead of made).
+template <int kMode, int kItems, bool kSeed, bool kOnce, bool kGrid>
+__global__ void __launch_bounds__(kAdvBlock, kItems == 1 ? 5 : kItems == 2 ? 4 : 2)
+    advec_kernel(oppb_advec_batch b, oppb_move_status* st, int32_t max_hops, int32_t chunk_items) {
     static_assert(kChunkItems % kItems == 0, "a chunk is a whole number of passes");
     static_assert(!kSeed || kMode != kUpdateOnly, "the seed belongs to the move");
     __shared__ int s_chunk;
@@ -180,9 +196,15 @@ __global__ void __launch_bounds__(kAdvBlock, kItems == 1 ? 5 : kItems == 2 ? 4 :
     int my_max = 0;
     int my_removed = 0;
     int cursor = 0;
-    int params_of = -1;  // the instance whose reciprocals these are
+    // What a block keeps of the instance it walks, where it has more than one chunk: a grid's 1 / nx and
+    // row count, and the extents' reciprocals where the registers allow.
+    constexpr bool kKept = kGrid && !kOnce;
+    constexpr int kWrap = kOnce ? kDivide : kMode == kUpdateOnly || (kGrid && !kSeed) ? kKeptReciprocal
+                                        : kGrid                                       ? kOwnReciprocal
+                                                                                      : kDivide;
+    int kept_of = -1;
     double inv_ex = 0.0, inv_ey = 0.0, inv_nx = 0.0;
-    int32_t gny = 0;
+    int32_t ny = 0;
     const int64_t sd = b.stride;
     for (;;) {
         int chunk = (int)blockIdx.x * chunk_items;
@@ -225,17 +247,16 @@ __global__ void __launch_bounds__(kAdvBlock, kItems == 1 ? 5 : kItems == 2 ? 4 :
                 const oppb_advec_instance& I = b.instances[inst[k]];
                 const int64_t i = idx[k];
                 const double ex = __ldg(&I.extents[0]), ey = __ldg(&I.extents[1]);
-                const int32_t gnx = __ldg(&I.grid_nx);
-                if (inst[k] != params_of) {
-                    params_of = inst[k];
-                    inv_ex = 1.0 / ex, inv_ey = 1.0 / ey;
-                    inv_nx = 1.0 / (double)(gnx > 0 ? gnx : 1);
-                    gny = gnx > 0 ? __ldg(&I.n_cells) / gnx : 0;
+                const int32_t nx = __ldg(&I.grid_nx);
+                if ((kKept || kWrap == kKeptReciprocal) && inst[k] != kept_of) {
+                    kept_of = inst[k];
+                    if (kWrap == kKeptReciprocal) inv_ex = 1.0 / ex, inv_ey = 1.0 / ey;
+                    if (kKept) inv_nx = 1.0 / (double)max(nx, 1), ny = __ldg(&I.n_cells) / max(nx, 1);
                 }
                 if (kMode != kMoveOnly) {
                     const double dt = __ldg(&I.dt);
-                    x[k] = update_axis(x[k], vx[k], dt, ex, inv_ex);
-                    y[k] = update_axis(y[k], vy[k], dt, ey, inv_ey);
+                    x[k] = update_axis<kWrap>(x[k], vx[k], dt, ex, inv_ex);
+                    y[k] = update_axis<kWrap>(y[k], vy[k], dt, ey, inv_ey);
                     st_stream(b.pos + i, x[k]);
                     st_stream(b.pos + sd + i, y[k]);
                 }
@@ -249,12 +270,20 @@ __global__ void __launch_bounds__(kAdvBlock, kItems == 1 ? 5 : kItems == 2 ? 4 :
                             continue;
                         }
                     }
-                    int err = 0, mx = 0, my = 0;
-                    const int calls =
-                        gnx > 0 ? move_particle_grid(gnx, gny, inv_nx, __ldg(&I.n_cells), x[k], y[k], mx, my, cell[k],
-                                                     __ldg(&I.cell_width), ex, ey, max_hops, err)
-                                : move_particle(b.cells, __ldg(&I.cell_offset), __ldg(&I.n_cells), x[k], y[k], mx, my,
-                                                cell[k], __ldg(&I.cell_width), ex, ey, max_hops, err);
+                    int err = 0, mx = 0, my = 0, calls = 0;
+                    const int32_t n_cells = __ldg(&I.n_cells);
+                    const double cw = __ldg(&I.cell_width);
+                    if (!kGrid && nx <= 0) {
+                        calls = move_particle(b.cells, __ldg(&I.cell_offset), n_cells, x[k], y[k], mx, my, cell[k], cw, ex, ey,
+                                              max_hops, err);
+                    } else if ((uint32_t)cell[k] >= (uint32_t)n_cells || nx <= 0) {
+                        err = OPPB_ERR_CELL_RANGE;
+                    } else {
+                        // (cell + 0.5) / nx is half a cell from an integer, so truncating the product gives cell / nx.
+                        const int32_t iy = kKept ? __double2int_rz(((double)cell[k] + 0.5) * inv_nx) : cell[k] / nx;
+                        calls = move_particle_grid(nx, kKept ? ny : n_cells / nx, iy, x[k], y[k], mx, my, cell[k], cw, ex, ey,
+                                                   max_hops, err);
+                    }
                     if (err) raise_error(st, err, (int32_t)i);
                     if (calls > 0) {  // without a call (an invalid cell) the direction stays as it was
                         st_stream(b.mdir + i, mx);
@@ -334,7 +363,7 @@ __global__ void __launch_bounds__(256) advec_check_grid_kernel(const double* cel
 }
 
 // Persistent grid: resident blocks of the kernel on every SM (cached per device and variant).
-template <int kMode, int kItems, bool kSeed>
+template <int kMode, int kItems, bool kSeed, bool kGrid>
 int resident_blocks() {
     static int cached[64] = {0};
     int dev = 0;
@@ -342,7 +371,7 @@ int resident_blocks() {
     if (!cached[dev]) {
         int sms = 0, per_sm = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, advec_kernel<kMode, kItems, kSeed, false>, kAdvBlock,
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, advec_kernel<kMode, kItems, kSeed, false, kGrid>, kAdvBlock,
                                                       0);
         cached[dev] = sms * (per_sm > 0 ? per_sm : 1);
     }
@@ -353,29 +382,29 @@ int resident_blocks() {
 // its index: no counter to reset, and 8-item chunks would leave most SMs idle (538 items of one
 // 61 x 61-cell instance: 14.6 us as 68 chunks of eight, 5.3 as 538 of one).  Larger batches go
 // through the counter.
-template <int kMode, int kItems, bool kSeed>
+template <int kMode, int kItems, bool kSeed, bool kGrid>
 int launch_items(const oppb_advec_batch* b, oppb_move_status* status, int32_t max_hops, cudaStream_t s) {
-    const int resident = resident_blocks<kMode, kItems, kSeed>();
+    const int resident = resident_blocks<kMode, kItems, kSeed, kGrid>();
     const int passes = ceil_div(b->n_work, kItems);
     if (passes <= resident) {
-        advec_kernel<kMode, kItems, kSeed, true><<<passes, kAdvBlock, 0, s>>>(*b, status, max_hops, kItems);
+        advec_kernel<kMode, kItems, kSeed, true, kGrid><<<passes, kAdvBlock, 0, s>>>(*b, status, max_hops, kItems);
         return OPPB_OK;
     }
     if (cudaMemsetAsync(b->work_counter, 0, sizeof(int32_t), s) != cudaSuccess) return OPPB_ERR_LAUNCH;
     const int chunks = ceil_div(b->n_work, kChunkItems);
     const int grid = resident > 0 && resident < chunks ? resident : chunks;
-    advec_kernel<kMode, kItems, kSeed, false><<<grid, kAdvBlock, 0, s>>>(*b, status, max_hops, kChunkItems);
+    advec_kernel<kMode, kItems, kSeed, false, kGrid><<<grid, kAdvBlock, 0, s>>>(*b, status, max_hops, kChunkItems);
     return OPPB_OK;
 }
 
-template <int kMode, bool kSeed>
+template <int kMode, bool kSeed, bool kGrid>
 int launch_seeded(const oppb_advec_batch* b, oppb_move_status* status, int32_t max_hops, cudaStream_t s) {
     const int items = tuning().advec_items;
     // One item a block while every item has a resident block.
-    if (items == 1 || b->n_work <= resident_blocks<kMode, 1, kSeed>())
-        return launch_items<kMode, 1, kSeed>(b, status, max_hops, s);
-    return items == 4 ? launch_items<kMode, 4, kSeed>(b, status, max_hops, s)
-                      : launch_items<kMode, 2, kSeed>(b, status, max_hops, s);
+    if (items == 1 || b->n_work <= resident_blocks<kMode, 1, kSeed, kGrid>())
+        return launch_items<kMode, 1, kSeed, kGrid>(b, status, max_hops, s);
+    return items == 4 ? launch_items<kMode, 4, kSeed, kGrid>(b, status, max_hops, s)
+                      : launch_items<kMode, 2, kSeed, kGrid>(b, status, max_hops, s);
 }
 
 // The pointers a launch reads or writes must be set: pos always, vel unless the launch only
@@ -420,7 +449,7 @@ __global__ void __launch_bounds__(256) advec_verify_kernel(const double* __restr
     if (threadIdx.x == 0 && s_bad) atomicAdd(incorrect, s_bad);
 }
 
-template <int kMode>
+template <int kMode, bool kGrid>
 int launch_advec(const oppb_advec_batch* b, oppb_move_status* status, int32_t max_hops, void* stream) {
     const int rc = check_batch<kMode>(b);
     if (rc) return rc;
@@ -429,10 +458,10 @@ int launch_advec(const oppb_advec_batch* b, oppb_move_status* status, int32_t ma
     cudaStream_t s = as_stream(stream);
     int rc2 = OPPB_OK;
     if constexpr (kMode != kUpdateOnly)
-        rc2 = b->dh ? launch_seeded<kMode, true>(b, status, max_hops, s)
-                    : launch_seeded<kMode, false>(b, status, max_hops, s);
+        rc2 = b->dh ? launch_seeded<kMode, true, kGrid>(b, status, max_hops, s)
+                    : launch_seeded<kMode, false, kGrid>(b, status, max_hops, s);
     else
-        rc2 = launch_seeded<kMode, false>(b, status, max_hops, s);
+        rc2 = launch_seeded<kMode, false, kGrid>(b, status, max_hops, s);
     if (rc2) return rc2;
     count_launches(1);
     return launch_status();
@@ -468,16 +497,16 @@ extern "C" int oppb_advec_check_grid(const double* cells, int32_t cell_offset, i
 
 extern "C" int oppb_advec_step(const oppb_advec_batch* batch, oppb_move_status* status, int32_t max_hops,
                                void* stream) {
-    return oppb::launch_advec<oppb::kStep>(batch, status, max_hops, stream);
+    return oppb::launch_advec<oppb::kStep, false>(batch, status, max_hops, stream);
 }
 
 extern "C" int oppb_advec_update_pos(const oppb_advec_batch* batch, void* stream) {
-    return oppb::launch_advec<oppb::kUpdateOnly>(batch, nullptr, 1, stream);
+    return oppb::launch_advec<oppb::kUpdateOnly, false>(batch, nullptr, 1, stream);
 }
 
 extern "C" int oppb_advec_move(const oppb_advec_batch* batch, oppb_move_status* status, int32_t max_hops,
                                void* stream) {
-    return oppb::launch_advec<oppb::kMoveOnly>(batch, status, max_hops, stream);
+    return oppb::launch_advec<oppb::kMoveOnly, false>(batch, status, max_hops, stream);
 }
 
 extern "C" int oppb_advec_verify(const double* pos, int64_t stride, const int32_t* p2c, const int32_t* c_gbl_idx,
@@ -490,4 +519,14 @@ extern "C" int oppb_advec_verify(const double* pos, int64_t stride, const int32_
                                                                               nx, cell_width, incorrect);
     count_launches(1);
     return launch_status();
+}
+
+extern "C" int oppb_advec_step_grid(const oppb_advec_batch* batch, oppb_move_status* status, int32_t max_hops,
+                                    void* stream) {
+    return oppb::launch_advec<oppb::kStep, true>(batch, status, max_hops, stream);
+}
+
+extern "C" int oppb_advec_move_grid(const oppb_advec_batch* batch, oppb_move_status* status, int32_t max_hops,
+                                    void* stream) {
+    return oppb::launch_advec<oppb::kMoveOnly, true>(batch, status, max_hops, stream);
 }

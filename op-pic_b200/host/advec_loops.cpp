@@ -180,7 +180,7 @@ void opp_particle_move__move_kernel(opp_set set, opp_map c2c_map, opp_map p2c_ma
     oppb_move_status* st = oppb_rt::move_status();
     check_cuda(cudaMemsetAsync(st, 0, sizeof(oppb_move_status), s), "status reset");
     const oppb_advec_batch b = batch_of(set, pos, nullptr, mdir);
-    check(oppb_advec_move(&b, st, oppb_rt::max_hops(), s), "oppb_advec_move");
+    check((adv().grid_nx > 0 ? oppb_advec_move_grid : oppb_advec_move)(&b, st, oppb_rt::max_hops(), s), "oppb_advec_move");
     if (b.dh)  // only the global move's pre-pass removes particles
         check(oppb_removal_bits(b.p2c, set->size, oppb_rt::remove_bits(set), s), "oppb_removal_bits");
     oppb_rt::mark_device_written(mdir);

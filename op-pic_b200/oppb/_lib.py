@@ -207,9 +207,11 @@ _SIGS = {
                                                  c_vp, c_i32, c_vp]),
     "oppb_advec_pack_cells": (C.c_int, [c_vp, c_i32, c_i32, c_i32, c_vp, c_vp, c_vp]),
     "oppb_advec_step": (C.c_int, [P(AdvecBatch), c_vp, c_i32, c_vp]),
+    "oppb_advec_step_grid": (C.c_int, [P(AdvecBatch), c_vp, c_i32, c_vp]),
     "oppb_advec_check_grid": (C.c_int, [c_vp, c_i32, c_i32, c_i32, C.c_double, c_vp, c_vp]),
     "oppb_advec_update_pos": (C.c_int, [P(AdvecBatch), c_vp]),
     "oppb_advec_move": (C.c_int, [P(AdvecBatch), c_vp, c_i32, c_vp]),
+    "oppb_advec_move_grid": (C.c_int, [P(AdvecBatch), c_vp, c_i32, c_vp]),
     "oppb_advec_verify": (C.c_int, [c_vp, c_i64, c_vp, c_vp, c_i32, c_i32, C.c_double, c_vp, c_vp]),
     "oppb_cabana_interpolate": (C.c_int, [c_i32, c_i64, c_vp, c_vp, P(c_vp), P(c_vp), c_vp, c_vp, c_vp]),
     "oppb_cabana_accumulate": (C.c_int, [c_i32, c_i64, c_vp, c_vp, P(c_vp), c_vp, P(C.c_double), c_vp]),

@@ -134,6 +134,7 @@ class AdvecBatchDevice:
                 if bad == 0:
                     self.grid_nx[k] = meshes[k].nx
                     table[k].grid_nx = meshes[k].nx
+        self.all_grid = all(self.grid_nx)
         self.instances = torch.frombuffer(bytearray(bytes(table)), dtype=torch.uint8).to(self.device)
         self.tile_prefix = torch.tensor(prefix, dtype=torch.int32, device=self.device)
         self.batch = L.AdvecBatch(len(meshes), prefix[-1], _ptr(self.instances), _ptr(self.tile_prefix),
@@ -214,15 +215,15 @@ class AdvecBatchDevice:
 
     def step(self, max_hops: int = 4096, stream=None) -> None:
         """update_pos + move of every instance, one persistent launch; status accumulates."""
-        L.check("oppb_advec_step", self.lib.oppb_advec_step(C.byref(self.batch), _ptr(self.status), max_hops,
-                                                            _stream(stream)))
+        fn = self.lib.oppb_advec_step_grid if self.all_grid else self.lib.oppb_advec_step
+        L.check("oppb_advec_step", fn(C.byref(self.batch), _ptr(self.status), max_hops, _stream(stream)))
 
     def update_pos(self, stream=None) -> None:
         L.check("oppb_advec_update_pos", self.lib.oppb_advec_update_pos(C.byref(self.batch), _stream(stream)))
 
     def move(self, max_hops: int = 4096, stream=None) -> None:
-        L.check("oppb_advec_move", self.lib.oppb_advec_move(C.byref(self.batch), _ptr(self.status), max_hops,
-                                                            _stream(stream)))
+        fn = self.lib.oppb_advec_move_grid if self.all_grid else self.lib.oppb_advec_move
+        L.check("oppb_advec_move", fn(C.byref(self.batch), _ptr(self.status), max_hops, _stream(stream)))
 
     def capture(self, steps: int, max_hops: int = 4096) -> torch.cuda.CUDAGraph:
         """A CUDA graph of `steps` consecutive step() launches.  Make one step() call first:
