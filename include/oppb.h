@@ -135,7 +135,10 @@ typedef struct oppb_tuning {
     int32_t deposit;     /* OPPB_DEPOSIT_* */
     int32_t replicas;    /* node-sum copies the deposit spreads its atomics over (1..64, default 8) */
     int32_t advec_items; /* NESO-advection step: 256-particle work items per block pass, i.e.
-                            particles per thread in flight (1, 2 or 4; default 2) */
+                            particles per thread in flight (1, 2 or 4; default 2).  A batch with no
+                            more items than blocks that fit the device at one item each (740 on a B200,
+                            189,000 particles) runs one a block whatever the value: more in flight a
+                            thread would leave SMs idle */
     int32_t sort_gather_cols; /* cell sort: particle-dat columns gathered per launch (1..16, default 16) */
     int32_t move_lanes;  /* lanes per particle of the FP64 move: 1 (0 reads as 1) = a particle per thread,
                             32 per warp; 2 = a particle per lane pair, 16 per warp, each lane reading one
