@@ -647,8 +647,7 @@ int launch_cabana(const oppb_hex_mesh* mesh, const oppb_cabana_particles* parts,
     auto kernel = occ == 5   ? cabana_move_deposit_kernel<kF32Mom, 5>
                   : occ == 4 ? cabana_move_deposit_kernel<kF32Mom, 4>
                              : cabana_move_deposit_kernel<kF32Mom, 0>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CabShared)) != cudaSuccess)
-        return OPPB_ERR_LAUNCH;
+    static_assert(sizeof(CabShared) <= 48 * 1024, "no attribute is needed for this much dynamic shared memory");
     kernel<<<ceil_div(parts->size, kCabBlock), kCabBlock, sizeof(CabShared), s>>>(
         m, p, *consts, kf, acc, acc_stride, status, max_hops);
     count_launches(1);
