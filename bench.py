@@ -50,7 +50,7 @@ BYTES_PER_NODE = 16
 # DRAM bytes per particle of one move+deposit launch (dram__bytes_read.sum + dram__bytes_write.sum),
 # from an ncu capture of full-size launches of this workload: profiles/move_mixed_kernel_fempic_48x48x192.txt
 # and profiles/move_f64_kernel_fempic_48x48x192.txt.
-MEASURED_DRAM_BYTES_PER_PARTICLE = {"f64": 73.0, "mixed": 70.0}
+MEASURED_DRAM_BYTES_PER_PARTICLE = {"f64": 72.6, "mixed": 70.0}
 TRAFFIC_SOURCE = "ncu dram__bytes_read.sum + dram__bytes_write.sum of full-size launches, per particle x particles"
 
 
@@ -825,7 +825,7 @@ CAB_WORKLOAD = ("CabanaPIC two-stream move + current deposit: 32x32x256 periodic
 CAB_BYTES_PER_PARTICLE = 108
 CAB_BYTES_PER_CELL = 384
 # DRAM bytes per particle of one full-size launch (ncu, profiles/cabana_move_deposit_kernel_twostream_32x32x256.txt).
-CAB_MEASURED_DRAM_BYTES_PER_PARTICLE = 122.0
+CAB_MEASURED_DRAM_BYTES_PER_PARTICLE = 122.8
 
 
 CAB_OCCUPANCY_CANDIDATES = [4, 0, 5]  # CTAs per SM the move + deposit kernel is compiled for (0: compiler's)
@@ -979,14 +979,13 @@ ADV = dict(instances=64, side_lo=64, side_hi=512, ppc_lo=10, ppc_hi=200, cell_wi
 ADV_WORKLOAD = ("NESO-advection ensemble: 64 independent periodic square meshes, side ~ U{64..512} cells, "
                 "10..200 particles per cell (seeded), |v dt| <= 0.5 cell per step; update_pos + move of every "
                 "instance in one persistent launch per step, captured as a CUDA graph")
-# Per step: read pos 16 + vel 16 + mdir 8 + p2c 4, write pos 16 + mdir 8 B per particle; 32 B per cell record.
-ADV_BYTES_PER_PARTICLE = 68
-ADV_BYTES_PER_CELL = 32
-# DRAM bytes per particle of one launch (ncu, profiles/advec_kernel_neso_ensemble_64.txt): a
-# 19.2M-particle, 8-instance capture, scaled by the particle count (traffic grows with it).
-ADV_MEASURED_DRAM_BYTES_PER_PARTICLE = 69.7
-ADV_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of an 8-instance, 19.2M-particle launch, "
-                      "per particle x particles")
+# Per step: read pos 16 + vel 16 + p2c 4, write pos 16 + mdir 8 + p2c 4 B per particle (the ensemble's
+# meshes are verified grids, whose cell records are not read).
+ADV_BYTES_PER_PARTICLE = 64
+# DRAM bytes per particle of one full-size launch (ncu, profiles/advec_kernel_neso_ensemble_64.txt).
+ADV_MEASURED_DRAM_BYTES_PER_PARTICLE = 64.3
+ADV_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of full-size launches, per particle x "
+                      "particles")
 
 
 def run_advec(dev, steps: int, warmup: int, cpu: bool, rank: int = 0, world: int = 1) -> dict:
@@ -1065,8 +1064,7 @@ def run_advec(dev, steps: int, warmup: int, cpu: bool, rank: int = 0, world: int
     direct, _ = replica_job_value(ps, t_direct, 0.0, dev)
     single, _ = replica_job_value(ps, t_single, 0.0, dev)
     n_all = int(round(replica_sum(float(n), dev)))
-    cells = sum(m.n_cells for m in meshes)
-    bytes_step = ADV_BYTES_PER_PARTICLE * n + ADV_BYTES_PER_CELL * cells
+    bytes_step = ADV_BYTES_PER_PARTICLE * n
     peaks = measured_peaks()
     achieved = bytes_step / (t_graph / graph_steps) / 1e9 if t_graph > 0 else 0.0
     out = {"workload": ADV_WORKLOAD, "metric": "particle-steps/s (update_pos + move, all instances)", "unit": UNIT,

@@ -108,9 +108,10 @@ int oppb_field_solve(const oppb_field_device* f, const oppb_field_consts* c, con
 
 /* How a solve is launched (oppb_field_solve: OPPB_FIELD_MAX_POLLS, 0).  max_polls bounds each wait among
  * the CG's blocks, in polls of about a microsecond; only the solve of a system by diagonals too
- * large for one cluster polls.  If a wait runs out, the step is not taken: D keeps its values,
- * node_potential is that of D, and the status says not converged.  no_cluster = 1 solves a small
- * system by diagonals as on a device that cannot place its cluster of blocks. */
+ * large for one cluster polls.  If a wait runs out, the step is not taken: D keeps its values (F1
+ * has its integrals added), node_potential is that of D, and the status says not converged.
+ * no_cluster = 1 solves a small system by diagonals as on a device that cannot place its cluster
+ * of blocks. */
 #define OPPB_FIELD_MAX_POLLS (1 << 20)
 typedef struct oppb_field_options {
     int32_t max_polls;

@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(kFieldBlock) field_newton_kernel(FieldArgs a) 
 //
 // What bounds the CG is neither DRAM nor arithmetic but what an iteration does one after the
 // other: grid barriers, passes over vectors in memory and the loads of K.  So each block owns a
-// contiguous range of rows and keeps x, r, q and the diagonal of its rows in registers, as many
+// contiguous range of rows and keeps x, r, z and the diagonal of its rows in registers, as many
 // diagonals of K as fit in shared memory (the others are streamed from L2), and the search
 // direction p of its rows and of the rows its diagonals reach in a shared-memory window.  Only
 // z = r / diag crosses blocks: every block forms p = z + beta p on its whole window itself (the
