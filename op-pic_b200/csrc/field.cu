@@ -307,7 +307,6 @@ constexpr int kCgMaxCluster = 16;
 constexpr int kCgMaxWarps = kCgMaxThreads / 32;
 constexpr int kCgMaxBlocks = 160;  // of the grid form
 
-
 // One block's sums in global memory: each value and the number of the reduction it belongs to are
 // one 16-byte word, so that a block that reads the number has the value too.  A slot fills a
 // 128-byte line: every block polls every slot, and packed slots would all be served by a few L2

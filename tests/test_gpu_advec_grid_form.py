@@ -1,7 +1,7 @@
 """The kernels for batches of grids only (oppb_advec_step_grid, oppb_advec_move_grid) against the general
 ones on the same state, bit for bit: sizes of one item a block and past the resident blocks, every
-number of items a pass, with and without the global move, extents at the limits of the wrap by a
-reciprocal, and an instance without a grid, which they refuse particle by particle."""
+number of items a pass, with and without the global move, quotients at and extents past the limits of
+the wrap by a reciprocal, and an instance without a grid, which they refuse particle by particle."""
 from __future__ import annotations
 
 import ctypes as C
@@ -86,6 +86,30 @@ def test_extents_past_fp32(cw, dh):
     _call(b, "step", True)
     torch.cuda.synchronize()
     assert torch.equal(a.pos.view(torch.int64), b.pos.view(torch.int64))
+
+
+@pytest.mark.parametrize("dh", [None, 0.7])
+@pytest.mark.parametrize("nx,ny,cw", [(13, 9, 0.7), (61, 61, 1.0), (5, 37, 0.25)])
+def test_quotients_next_to_integers(nx, ny, cw, dh):
+    """Multiples of the extents, a few ulps and up to 2^-18 around them, where the divide decides or takes
+    over from the reciprocal, in batches of more than one wave (one wave always divides)."""
+    m = AdvecMesh(nx, ny, cw)
+    rng = np.random.default_rng(nx)
+    n = 1300 * 256
+    away = [0.0, 1e-16, -1e-16, 3e-7, -3e-7, 2.0 ** -20, -2.0 ** -20, 2e-6, -3e-6, 0.5]
+    pos = (rng.integers(-3, 4, (n, 2)) + rng.choice(away, (n, 2))) * np.array(m.extents)
+    for _ in range(3):
+        step = rng.integers(-1, 2, (n, 2))
+        pos = np.where(step > 0, np.nextafter(pos, np.inf), np.where(step < 0, np.nextafter(pos, -np.inf), pos))
+    host = [(pos, np.zeros((n, 2)), np.full((n, 2), 7, np.int32), rng.integers(0, m.n_cells, n).astype(np.int32))]
+    a, b = _pair([m], host, [0.5], dh)
+    _call(a, "step", False)
+    _call(b, "step", True)
+    _same(a, b)
+    c, _ = _pair([m], host, [0.5])
+    c.update_pos()
+    torch.cuda.synchronize()
+    assert torch.equal(c.pos.view(torch.int64), b.pos.view(torch.int64))
 
 
 @pytest.mark.parametrize("ppc", [3, 90])

@@ -1,6 +1,6 @@
-"""The advection step's wrap without a divide and its launch shapes: positions whose quotient by the
-extent is an integer or next to one (the exact divide decides there), far outside the extents
-and on cell edges; batches of one item a block, of several, and past the resident blocks.
+"""The advection step's wrap and its launch shapes: positions whose quotient by the extent is an integer
+or next to one, far outside the extents and on cell edges (in one wave, which divides; the wrap by
+reciprocals of larger batches is in test_gpu_advec_grid_form); batches of one item a block, of several, and past the resident blocks.
 Positions, directions and cells bit-exact with the oracle."""
 from __future__ import annotations
 
